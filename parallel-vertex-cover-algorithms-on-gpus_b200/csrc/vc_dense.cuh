@@ -26,6 +26,9 @@
 //    recounted, one vertex per lane;
 //  * the triangle test of a degree-2 vertex is one bit test and the leaf
 //    rule's neighbour one find-first-set: no serial CSR row walks;
+//  * a node's children are bounded by a clique packing before either is entered
+//    ("the packing bound" below): a closed child costs no node, and with one
+//    left the node is no branch;
 //  * backtracking: an undo trail of removed ids (u16) and frames of (trail
 //    position, branching vertex); restoring ORs bits back into L.
 //
@@ -34,6 +37,8 @@
 #include "vc_search.cuh"
 
 namespace vcg {
+
+__device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 template <int NW>
 struct Rows {
@@ -122,7 +127,6 @@ struct DSU {
 
 enum : uint32_t { kPendApply = 1, kPendRecount = 2 };
 
-__device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 template <int NW>
 __device__ __forceinline__ void dsu_bind(DSU<NW> &s, uint8_t *ws, const uint32_t *adj)
@@ -314,6 +318,219 @@ __device__ __forceinline__ void dense_restore(DSU<NW> &s, uint32_t pos)
     s.stat.restored += s.top - pos;
     s.top = pos;
     __syncwarp();
+}
+
+// ---- the packing bound
+// What a node still needs is bounded from below by vertex-disjoint cliques of its
+// live graph, of which any cover takes all vertices but one.  They are picked
+// greedily: a vertex of least degree among the unpicked, its neighbour of least
+// degree, and common neighbours of all picked so far while there are any.
+// The degrees among the unpicked are held bit-sliced, plane B[k] having bit k of
+// each degree and lane w the 32 vertices of word w, so that a row is taken off
+// all degrees by one borrow chain.  Graphs of up to 512 vertices fill half a warp
+// at most, so a warp bounds two nodes in step, one per group of 16 lanes.
+// A step is a chain of four ballots, two shuffles and two row loads, about a
+// hundred instructions, and a bound takes some forty of them: it is what a node
+// now spends most of its time on, bound by issue with the SM full and by that
+// chain's latency without.  It pays for itself many times over: 512 graphs of 30
+// to 160 vertices and average degree 3 to 12 in one batch take 1.6 M nodes and
+// 32 ms instead of 161 M and 470 ms; one of 197 vertices and 648 edges 16 k and
+// 1.6 ms instead of 3.6 M and 22 ms.  Degrees bit-sliced rather than in bytes
+// (four to a word, a word per lane) took the 512 graphs from 66 to 49 ms, and
+// bounding both children of a node instead of each node as it is reached to 32.
+constexpr int kPackPlanes = 5;  // degrees below 32
+constexpr uint32_t kPackNow = 1u << 31;  // beside InstState's flags in a unit's copy: the bound's time has come
+
+template <int NW>
+struct PackGroup {
+    static constexpr uint32_t kLanes = NW <= 16 ? 16 : 32;
+    static constexpr uint32_t kGroups = 32 / kLanes;
+    // This group's bits of a ballot, and its share of a warp-wide sum (below 2^16 per group).
+    static __device__ __forceinline__ uint32_t of(uint32_t bal)
+    {
+        return kGroups == 1 ? bal : (bal >> (lane_id() & 16u)) & 0xffffu;
+    }
+    static __device__ __forceinline__ uint32_t sum(uint32_t x)
+    {
+        if constexpr (kGroups == 1) return __reduce_add_sync(0xffffffffu, x);
+        else return (__reduce_add_sync(0xffffffffu, x << (lane_id() & 16u)) >> (lane_id() & 16u)) & 0xffffu;
+    }
+};
+
+// The lowest vertex of the sets e (a word per lane, at least one bit in this
+// lane's group unless the group is done): adds it to `picked` and returns its
+// row's word among the live.
+template <int NW>
+__device__ __forceinline__ uint32_t pack_pick(const uint32_t *adj, uint32_t e, uint32_t bal, uint32_t word, uint32_t live,
+                                              uint32_t &picked)
+{
+    using PG = PackGroup<NW>;
+    const uint32_t src = bal ? __ffs(bal) - 1 : 0u;  // the word it is in
+    const uint32_t bit = word == src ? e & (0u - e) : 0u;
+    picked |= bit;
+    const uint32_t at = PG::kGroups == 1 ? src : src + (lane_id() & 16u);
+    const uint32_t v = 32u * src + (31u - __clz(__shfl_sync(0xffffffffu, bit, at) | 1u));
+    return adj[Rows<NW>::at(v, word < (uint32_t)NW ? word : 0u)] & live;
+}
+
+// Takes the rows of the set bits `br` off the degrees.
+__device__ __forceinline__ void pack_subtract(uint32_t (&B)[kPackPlanes], uint32_t br)
+{
+#pragma unroll
+    for (int k = 0; k < kPackPlanes; ++k) {
+        const uint32_t t = B[k];
+        B[k] = t ^ br;
+        br &= ~t;
+    }
+}
+
+// True for the lanes of a group whose graph (planes B, this lane's word of its
+// vertices) needs more than `b` vertices (b < 0: always).  Stops as soon as the
+// packing says so, or as soon as that looks out of reach: a vertex of degree d is
+// in a clique of at most d + 1 vertices and only one on a triangle of the staged
+// graph in one of more than two, so what is left is taken to be worth half a
+// vertex to each, two thirds if it is in tri, and then five sixths from degree 3
+// and one from degree 6.
+template <int NW>
+__device__ __forceinline__ bool packing_exceeds(const uint32_t *adj, uint32_t (&B)[kPackPlanes], int32_t b, uint32_t tri)
+{
+    using PG = PackGroup<NW>;
+    constexpr int K = kPackPlanes;
+    const uint32_t word = lane_id() & (PG::kLanes - 1u);
+    const int32_t need = 6 * (b + 1);
+    int32_t have = 0;
+    bool over = b < 0, go = !over;
+    uint32_t live = B[0] | B[1] | B[2] | B[3] | B[4];  // unpicked with an unpicked neighbour
+    for (int it = 0; it < 16 * NW; ++it) {  // a group's step picks two vertices at least
+        uint32_t bal4 = PG::of(__ballot_sync(0xffffffffu, live != 0u));
+        go = go && bal4 != 0u;
+        if ((it & 3) == 0) {
+            const uint32_t t = live & tri, three = B[2] | B[3] | B[4] | (B[1] & B[0]), six = B[3] | B[4] | (B[2] & B[1]);
+            const int32_t left =
+                (int32_t)PG::sum(3u * __popc(live) + __popc(t) + __popc(t & three) + __popc(t & six));
+            go = go && have + left >= need;
+        }
+        if (!__any_sync(0xffffffffu, go)) break;
+        // degrees 1, 2, 3 and the rest
+        const uint32_t hi = B[2] | B[3] | B[4];
+        const uint32_t c1 = B[0] & ~(B[1] | hi), c2 = B[1] & ~(B[0] | hi), c3 = B[0] & B[1] & ~hi;
+        const uint32_t bal1 = PG::of(__ballot_sync(0xffffffffu, c1 != 0u));
+        uint32_t bal2 = PG::of(__ballot_sync(0xffffffffu, c2 != 0u));
+        uint32_t bal3 = PG::of(__ballot_sync(0xffffffffu, c3 != 0u));
+        uint32_t picked = 0u;
+        const uint32_t nu = pack_pick<NW>(adj, bal1 ? c1 : (bal2 ? c2 : (bal3 ? c3 : live)),
+                                          bal1 ? bal1 : (bal2 ? bal2 : (bal3 ? bal3 : bal4)), word, live, picked);
+        // its neighbour of the lowest class
+        bal2 = PG::of(__ballot_sync(0xffffffffu, (nu & c2) != 0u));
+        bal3 = PG::of(__ballot_sync(0xffffffffu, (nu & c3) != 0u));
+        bal4 = PG::of(__ballot_sync(0xffffffffu, nu != 0u));
+        const uint32_t np = pack_pick<NW>(adj, nu & (bal2 ? c2 : (bal3 ? c3 : ~0u)), bal2 ? bal2 : (bal3 ? bal3 : bal4), word,
+                                          live, picked);
+        have += 6;
+        // common neighbours, as long as there are any
+        const uint32_t unpicked = live;
+        uint32_t common = nu & np;
+        for (int more = 0; more < 32; ++more) {
+            const uint32_t any = __ballot_sync(0xffffffffu, common != 0u);
+            if (!any) break;
+            const uint32_t bal = PG::of(any);
+            const uint32_t row = pack_pick<NW>(adj, common, bal, word, bal ? unpicked : 0u, picked);
+            pack_subtract(B, row);
+            common &= row;
+            have += bal ? 6 : 0;
+        }
+        if (go && have >= need) { over = true; go = false; }
+        // the degrees less the first two rows (their sum in two bits, then a borrow chain)
+        const uint32_t s0 = nu ^ np, s1 = nu & np;
+        uint32_t br = ~B[0] & s0;
+        B[0] = (B[0] ^ s0) & ~picked;
+        const uint32_t b1 = B[1];
+        B[1] = (b1 ^ s1 ^ br) & ~picked;
+        br = (~b1 & (s1 | br)) | (s1 & br);
+        live = B[0] | B[1];
+#pragma unroll
+        for (int k = 2; k < K; ++k) {
+            const uint32_t bk = B[k];
+            B[k] = (bk ^ br) & ~picked;
+            br &= ~bk;
+            live |= B[k];
+        }
+        if (!go) live = 0u;  // this group is done: its lanes only keep the other one company
+    }
+    return over;
+}
+
+// Which children of a settled node on vertex v the packing bound leaves open,
+// when b more vertices may be taken: bit 0 "take v", bit 1 "take N(v)".  The
+// children are bounded before their own reductions (picking vertices of degree 1
+// first does for the bound what the leaf rule does for the node), so a child
+// that is closed costs no settling, and a node with one open child is not a
+// branch.  Needs degrees below 2^kPackPlanes.
+template <int NW>
+__device__ __forceinline__ uint32_t open_children(DSU<NW> &s, uint32_t v, uint32_t maxd, uint32_t b)
+{
+    using PG = PackGroup<NW>;
+    constexpr int J = Rows<NW>::kJ;
+    constexpr bool H = Rows<NW>::kHalf;
+    constexpr int K = kPackPlanes;
+    const unsigned lane = lane_id();
+    const uint32_t word = lane & (PG::kLanes - 1u);
+    uint32_t *d32 = reinterpret_cast<uint32_t *>(s.degs());
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const uint32_t q = 32u * j + lane;
+        if (q < (H ? 16u : 8u) * s.nw) d32[q] = s.D[j];
+    }
+    __syncwarp();
+    uint32_t A[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) A[k] = 0u;
+#pragma unroll 1
+    for (uint32_t w = 0; w < s.nw; ++w) {
+        const uint32_t d = H ? s.degs16()[32u * w + lane] : s.degs()[32u * w + lane];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t x = __ballot_sync(0xffffffffu, (d >> k) & 1u);
+            if (word == w) A[k] = x;
+        }
+    }
+    const uint32_t live = A[0] | A[1] | A[2] | A[3] | A[4];
+    const uint32_t at = word < (uint32_t)NW ? word : 0u;
+    const uint32_t tri = word < (uint32_t)NW ? s.adj[Rows<NW>::kTri + at] : 0u;
+    const uint32_t nv = s.adj[Rows<NW>::at(v, at)] & live;
+    const uint32_t vbit = word == (v >> 5) ? 1u << (v & 31u) : 0u;
+    uint32_t open = 0;
+#pragma unroll 1
+    for (uint32_t side = 0; side < 2; side += PG::kGroups) {
+        const bool right = PG::kGroups == 2 ? lane >= 16u : side != 0u;  // this group's child takes N(v)
+        uint32_t B[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) B[k] = A[k];
+        const uint32_t gone = right ? nv | vbit : vbit;
+        if (PG::kGroups == 2 || !right) {  // v's row comes off in the left child
+            pack_subtract(B, right ? 0u : nv);
+        }
+        if (PG::kGroups == 2 || right) {  // the rows of v's neighbours in the right child
+            uint32_t wm = PG::of(__ballot_sync(0xffffffffu, nv != 0u));
+            while (wm) {
+                const uint32_t w = __ffs(wm) - 1;
+                wm &= wm - 1;
+                uint32_t m = __shfl_sync(0xffffffffu, nv, w);
+                while (m) {
+                    const uint32_t u = 32u * w + (__ffs(m) - 1);
+                    m &= m - 1;
+                    pack_subtract(B, right ? s.adj[Rows<NW>::at(u, at)] & live : 0u);
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) B[k] &= ~gone;
+        const int32_t bc = (int32_t)b - (right ? (int32_t)maxd : 1);
+        const uint32_t closed = __ballot_sync(0xffffffffu, packing_exceeds<NW>(s.adj, B, bc, tri));
+        if constexpr (PG::kGroups == 2) open = ((closed & 1u) ^ 1u) | (((closed >> 16) & 1u) ^ 1u) << 1;
+        else open |= ((closed & 1u) ^ 1u) << side;
+    }
+    return open;
 }
 
 // The set in s.marks() has just left L (trail, L and its mirror already
@@ -973,6 +1190,13 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
     uint32_t ticks = 0, c_flags = 0;
     unsigned long long c_state = 0;
     const unsigned lane = lane_id();
+    // How often the incumbent and the idle units are looked up: a plain solve's
+    // tree is over in a few hundred nodes per unit, so every other node (against
+    // every eighth: graphs of 175 and 197 vertices 0.65 and 1.62 -> 0.62 and 1.43 ms);
+    // a batch loses by it (1024 graphs 151 -> 162 ms).
+    const uint32_t tick_mask = P.count == 1 ? 1u : 7u;
+    bool packing = P.pack_after_ns == 0;
+    const unsigned long long t_pack = globaltimer() + P.pack_after_ns;
 
     for (;;) {
         if (!have) {
@@ -1000,7 +1224,7 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
             }
         }
         InstState &st = P.st[s.inst];
-        if ((ticks & 7u) == 0u) {
+        if ((ticks & tick_mask) == 0u) {
             uint32_t b = 0, f = 0;
             unsigned long long w = 0;
             if (lane == 0) {
@@ -1011,10 +1235,12 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
                     if (ld_relaxed_u64(&P.ctl[kAbort])) f |= kError;
                     else if (globaltimer() > s.deadline) { atomicExch(&P.ctl[kAbort], 1ull); f |= kError; }
                 }
+                if (!packing && globaltimer() > t_pack) f |= kPackNow;
             }
             s.c_best = G::bcast(b);
             c_flags = G::bcast(f);
             c_state = G::bcast64(w);
+            packing = packing || (c_flags & kPackNow);
         }
         ++ticks;
         if (c_flags & (kFound | kBudget | kError | kBadGraph)) {
@@ -1044,19 +1270,12 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
         if (kPhaseTimers && s.timed) s.cyc.scan += (unsigned long long)(clock64() - t_scan) - (s.cyc.apply - apply0);
         const uint32_t del = s.base_del + s.top;
         const uint64_t edges = o.sum / 2;
-        bool prune;
-        if (s.mode == kModeMVC) {
-            prune = del >= best;
-            if (!prune) {
-                uint64_t b = (uint64_t)(best - del - 1);
-                prune = edges >= b * b + 1;
-            }
-        } else {
-            prune = del > s.k;
-            if (!prune) {
-                uint64_t b = (uint64_t)(s.k - del);
-                prune = edges >= b * b + 1;
-            }
+        // b more vertices may be taken below this node
+        const uint32_t limit = s.mode == kModeMVC ? best - 1u : s.k;
+        bool prune = s.mode == kModeMVC ? del >= best : del > s.k;
+        if (!prune) {
+            const uint64_t b = (uint64_t)(limit - del);
+            prune = edges >= b * b + 1 || edges > b * o.maxd;
         }
         if (prune) { have = false; continue; }
         if (o.maxd == 0) {
@@ -1064,29 +1283,45 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
             have = false;
             continue;
         }
-        const long long t_br = (kPhaseTimers && s.timed) ? clock64() : 0;
         const uint32_t v = o.amax;
-        if (lane == 0) s.frames()[s.fr_top] = (s.top << 16) | v;
-        s.fr_top += 1;
-        __syncwarp();
-        uint32_t want = 0;
-        if (lane == 0) {
-            uint32_t li = vld(&cp.hdr[kCpIdle]), lc = vld(&cp.hdr[kCpCount]);
-            const bool local_need = li > lc;
-            const bool ring_need = (long long)(uint32_t)c_state - (long long)(c_state >> 32) > (long long)P.ring_bias;
-            // both a sibling warp and another CTA wait: the policy decides (local
-            // first, ring first, or alternating)
-            if (local_need && ring_need)
-                want = (P.ring_first == 1 || (P.ring_first == 2 && (s.stat.donations & 1ull))) ? 2 : 1;
-            else if (local_need) want = 1;
-            else if (ring_need) want = 2;
+        // Degrees of at most 2 leave disjoint cycles (the leaf rule took the paths),
+        // and every vertex of a cycle is in one of its minimum covers: no branch.
+        const uint32_t open = o.maxd == 2u ? 1u
+                              : packing && o.maxd < (1u << kPackPlanes)
+                                  ? open_children(s, v, o.maxd, limit - del)
+                                  : 3u;
+        if (open == 0u) { have = false; continue; }
+        const long long t_br = (kPhaseTimers && s.timed) ? clock64() : 0;
+        if (open == 3u) {  // a branch: "take N(v)" waits in a frame
+            if (lane == 0) s.frames()[s.fr_top] = (s.top << 16) | v;
+            s.fr_top += 1;
+            __syncwarp();
         }
-        want = G::bcast(want);
-        if (want == 1) donate_local<G, S>(s, P, cp);
-        else if (want == 2 && donate_global<G, S>(s, P)) c_state += 1ull << 32;
-        if (lane == 0) s.marks()[v >> 5] = 1u << (v & 31u);  // marks are clear after a settled node
+        if (s.fr_top > s.fr_bot) {  // a waiting child to give away, at a node that does not branch too
+            uint32_t want = 0;
+            if (lane == 0) {
+                uint32_t li = vld(&cp.hdr[kCpIdle]), lc = vld(&cp.hdr[kCpCount]);
+                const bool local_need = li > lc;
+                const bool ring_need = (long long)(uint32_t)c_state - (long long)(c_state >> 32) > (long long)P.ring_bias;
+                // both a sibling warp and another CTA wait: the policy decides (local
+                // first, ring first, or alternating)
+                if (local_need && ring_need)
+                    want = (P.ring_first == 1 || (P.ring_first == 2 && (s.stat.donations & 1ull))) ? 2 : 1;
+                else if (local_need) want = 1;
+                else if (ring_need) want = 2;
+            }
+            want = G::bcast(want);
+            if (want == 1) donate_local<G, S>(s, P, cp);
+            else if (want == 2 && donate_global<G, S>(s, P)) c_state += 1ull << 32;
+        }
+        // the child takes v, or N(v) where only that is left (marks are clear after a settled node)
+        if (open == 2u) {
+            if (lane < NW) s.marks()[lane] = s.adj[Rows<NW>::at(v, lane)] & s.lsm()[lane];
+        } else if (lane == 0) {
+            s.marks()[v >> 5] = 1u << (v & 31u);
+        }
         __syncwarp();
-        s.pending = kPendApply;  // the child takes v
+        s.pending = kPendApply;
         if (kPhaseTimers && s.timed) s.cyc.branch += (unsigned long long)(clock64() - t_br);
     }
     if (P.stats && lane == 0) {

@@ -1156,20 +1156,13 @@ __device__ void su_main(const Params &P, uint8_t *ws, CtaPool &cp)
             del = s.base_del + s.ctr[0];
         }
         del = s.base_del + s.ctr[0];
-        uint64_t edges = o.sum / 2;
-        bool prune;
-        if (s.mode == kModeMVC) {
-            prune = del >= best;
-            if (!prune) {
-                uint64_t b = (uint64_t)(best - del - 1);
-                prune = edges >= b * b + 1;
-            }
-        } else {
-            prune = del > s.k;
-            if (!prune) {
-                uint64_t b = (uint64_t)(s.k - del);
-                prune = edges >= b * b + 1;
-            }
+        // b more vertices may be taken below this node, each of at most maxd edges
+        const uint64_t edges = o.sum / 2;
+        const uint32_t limit = s.mode == kModeMVC ? best - 1u : s.k;
+        bool prune = s.mode == kModeMVC ? del >= best : del > s.k;
+        if (!prune) {
+            const uint64_t b = (uint64_t)(limit - del);
+            prune = edges >= b * b + 1 || edges > b * o.maxd;
         }
         if (prune) { have = false; continue; }
         if (o.maxd == 0) {
@@ -1177,30 +1170,36 @@ __device__ void su_main(const Params &P, uint8_t *ws, CtaPool &cp)
             have = false;
             continue;
         }
-        // branch: push the N(v) child, continue with the v child
+        // branch: push the N(v) child, continue with the v child.  Degrees of at
+        // most 2 leave disjoint cycles (the leaf rule took the paths), and every
+        // vertex of a cycle is in one of its minimum covers: take v without a branch
         const uint32_t v = o.amax;
-        if (G::rank() == 0) {
-            s.fpos[s.fr_top] = s.ctr[0];
-            s.fv[s.fr_top] = v;
+        if (o.maxd > 2u) {
+            if (G::rank() == 0) {
+                s.fpos[s.fr_top] = s.ctr[0];
+                s.fv[s.fr_top] = v;
+            }
+            s.fr_top += 1;
+            G::sync();
         }
-        s.fr_top += 1;
-        G::sync();
         // share the shallowest pending child with starving siblings, else with idle CTAs
-        uint32_t want = 0;
-        if (G::rank() == 0) {
-            uint32_t li = vld(&cp.hdr[kCpIdle]), lc = vld(&cp.hdr[kCpCount]);
-            const bool local_need = li > lc;
-            const bool ring_need = (long long)(uint32_t)c_state - (long long)(c_state >> 32) > (long long)P.ring_bias;
-            // both a sibling warp and another CTA wait: the policy decides (local
-            // first, ring first, or alternating)
-            if (local_need && ring_need)
-                want = (P.ring_first == 1 || (P.ring_first == 2 && (s.stat.donations & 1ull))) ? 2 : 1;
-            else if (local_need) want = 1;
-            else if (ring_need) want = 2;
+        if (s.fr_top > s.fr_bot) {
+            uint32_t want = 0;
+            if (G::rank() == 0) {
+                uint32_t li = vld(&cp.hdr[kCpIdle]), lc = vld(&cp.hdr[kCpCount]);
+                const bool local_need = li > lc;
+                const bool ring_need = (long long)(uint32_t)c_state - (long long)(c_state >> 32) > (long long)P.ring_bias;
+                // both a sibling warp and another CTA wait: the policy decides (local
+                // first, ring first, or alternating)
+                if (local_need && ring_need)
+                    want = (P.ring_first == 1 || (P.ring_first == 2 && (s.stat.donations & 1ull))) ? 2 : 1;
+                else if (local_need) want = 1;
+                else if (ring_need) want = 2;
+            }
+            want = G::bcast(want);
+            if (want == 1) donate_local<G, SU>(s, P, cp);
+            else if (want == 2 && donate_global<G, SU>(s, P)) c_state += 1ull << 32;
         }
-        want = G::bcast(want);
-        if (want == 1) donate_local<G, SU>(s, P, cp);
-        else if (want == 2 && donate_global<G, SU>(s, P)) c_state += 1ull << 32;
         take_vertex<G>(s, v);
     }
     if (P.stats && G::rank() == 0) {
