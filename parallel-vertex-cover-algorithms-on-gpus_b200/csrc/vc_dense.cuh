@@ -1154,7 +1154,7 @@ __device__ bool acquire_cta(DSU<NW> &s, const Params &P, CtaPool &cp, uint32_t *
             __syncwarp();
             if (lane == 0) {
                 __threadfence();
-                st_release_u64(&P.pool_seq[slot_i], qpos + P.q_mask + 1);
+                ring_release(P, qpos);
             }
             if (start_record<G, S>(s, P)) return true;
             if (lane == 0) { __threadfence_block(); atomicAdd(&cp.hdr[kCpIdle], 1u); }

@@ -35,7 +35,7 @@
 //    that takes a record recounts its degrees from the bitmap.  Only a fully
 //    idle CTA changes graphs: next root from the cursor, else a ring record;
 //    termination is the (pending records, idle CTAs) word of vc_search.cuh;
-//  * bounded waits only: ring claims give up, idle loops and the node loop
+//  * bounded waits only: ring waits have a limit, idle loops and the node loop
 //    read %globaltimer against the launch's time limit.
 #pragma once
 #include "vc_dense.cuh"
@@ -697,7 +697,7 @@ __device__ void lanes_main(const Params &P, uint32_t *sm, uint32_t *hdr)
                 if (lane == 0) {
                     if (res == 2) {
                         __threadfence();
-                        st_release_u64(&P.pool_seq[qpos & P.q_mask], qpos + P.q_mask + 1);
+                        ring_release(P, qpos);
                     } else {
                         roots += 1;
                     }
@@ -928,9 +928,7 @@ __device__ void lanes_main(const Params &P, uint32_t *sm, uint32_t *hdr)
                 unsigned long long qpos = 0;
                 uint32_t ok = 0;
                 if (lane == 0) {
-                    atomicAdd(&P.ctl[kState], 1ull << 32);
                     if (ring_claim_enq(P, qpos)) ok = 1;
-                    else atomicAdd(&P.ctl[kState], 0xffffffff00000000ull);
                 }
                 ok = __shfl_sync(FULL, ok, 0);
                 if (ok) {
@@ -943,7 +941,7 @@ __device__ void lanes_main(const Params &P, uint32_t *sm, uint32_t *hdr)
                         __stcg(&slot[0], g);
                         lane_donate<NW, NT>(m, L, top, fbot, gnw, slot + 4, true);
                         __threadfence();
-                        st_release_u64(&P.pool_seq[qpos & P.q_mask], qpos + 1);
+                        ring_publish(P, qpos);
                         n_don += 1;
                     }
                     __syncwarp();

@@ -101,9 +101,7 @@ __device__ __forceinline__ bool mcm_donate(const Params &P, const McmArgs &A, In
     unsigned long long qpos = 0;
     uint32_t ok = 0;
     if (lane == 0) {
-        atomicAdd(&P.ctl[kState], 1ull << 32);
         if (ring_claim_enq(P, qpos)) ok = 1;
-        else atomicAdd(&P.ctl[kState], 0xffffffff00000000ull);
     }
     if (!__shfl_sync(0xffffffffu, ok, 0)) return false;
     qpos = __shfl_sync(0xffffffffu, qpos, 0);
@@ -126,7 +124,7 @@ __device__ __forceinline__ bool mcm_donate(const Params &P, const McmArgs &A, In
     __syncwarp();
     if (lane == 0) {
         __threadfence();
-        st_release_u64(&P.pool_seq[qpos & P.q_mask], qpos + 1);
+        ring_publish(P, qpos);
     }
     return true;
 }
@@ -169,7 +167,7 @@ __device__ __forceinline__ bool mcm_acquire(const Params &P, const McmArgs &A, I
             __syncwarp();
             if (lane == 0) {
                 __threadfence();
-                st_release_u64(&P.pool_seq[slot_i], qpos + P.q_mask + 1);
+                ring_release(P, qpos);
             }
             return true;
         }

@@ -646,37 +646,60 @@ __device__ __forceinline__ void load_root(SU &s)
 }
 
 // ---------------------------------------------------------------- global ring
-// Bounded MPMC ring (per-slot sequence numbers).  Both claims give up after a
-// few attempts instead of spinning: a failed claim is retried by the caller
-// after a back-off.
-__device__ __forceinline__ bool ring_claim_enq(const Params &P, unsigned long long &pos_out)
+// Bounded MPMC ring.  Places are handed out by fetch-and-add tickets, to a
+// producer against the pending count and to a consumer against the count of
+// published records, so any number of either gets one in a single round trip;
+// claiming head and tail by compare-and-swap let one unit through per round trip
+// to L2 (about 1.4 records/us), which left most of the chip idle once subtrees
+// had become a dozen nodes long.  The slots' sequence numbers order a slot's
+// writer and reader: waits on them are for a copy another unit has in progress,
+// and they are bounded; one that runs out stops the launch.
+constexpr int kRingSpins = 1 << 20;
+
+__device__ __forceinline__ bool ring_wait(const Params &P, unsigned long long pos, unsigned long long seq)
 {
-    for (int it = 0; it < 8; ++it) {
-        unsigned long long pos = ld_relaxed_u64(&P.ctl[kTail]);
-        unsigned long long seq = ld_acquire_u64(&P.pool_seq[pos & P.q_mask]);
-        long long dif = (long long)(seq - pos);
-        if (dif == 0) {
-            if (atomicCAS(&P.ctl[kTail], pos, pos + 1) == pos) { pos_out = pos; return true; }
-        } else if (dif < 0) {
-            return false;  // full
-        }
+    for (int it = 0; it < kRingSpins; ++it) {
+        if (ld_acquire_u64(&P.pool_seq[pos & P.q_mask]) == seq) return true;
+        __nanosleep(32);
     }
+    atomicExch(&P.ctl[kAbort], 1ull);
     return false;
 }
 
+// A place for one more record, counted as pending from here on; false (and not
+// counted) if half of the ring is pending.
+__device__ __forceinline__ bool ring_claim_enq(const Params &P, unsigned long long &pos_out)
+{
+    if ((atomicAdd(&P.ctl[kState], 1ull << 32) >> 32) > P.q_mask / 2) {
+        atomicAdd(&P.ctl[kState], 0xffffffff00000000ull);
+        return false;
+    }
+    pos_out = atomicAdd(&P.ctl[kTail], 1ull);
+    return ring_wait(P, pos_out, pos_out);
+}
+
+// The record at `pos` is written (by this thread, or before a barrier it passed).
+__device__ __forceinline__ void ring_publish(const Params &P, unsigned long long pos)
+{
+    st_release_u64(&P.pool_seq[pos & P.q_mask], pos + 1);
+    atomicAdd(&P.ctl[kAvail], 1ull);
+}
+
+// A published record to read; its slot goes back with ring_release.
 __device__ __forceinline__ bool ring_claim_deq(const Params &P, unsigned long long &pos_out)
 {
-    for (int it = 0; it < 2; ++it) {
-        unsigned long long pos = ld_relaxed_u64(&P.ctl[kHead]);
-        unsigned long long seq = ld_acquire_u64(&P.pool_seq[pos & P.q_mask]);
-        long long dif = (long long)(seq - (pos + 1));
-        if (dif == 0) {
-            if (atomicCAS(&P.ctl[kHead], pos, pos + 1) == pos) { pos_out = pos; return true; }
-        } else if (dif < 0) {
-            return false;  // empty, or the producer has not published yet
-        }
+    if ((long long)ld_relaxed_u64(&P.ctl[kAvail]) <= 0) return false;
+    if ((long long)atomicAdd(&P.ctl[kAvail], ~0ull) <= 0) {  // others were first
+        atomicAdd(&P.ctl[kAvail], 1ull);
+        return false;
     }
-    return false;
+    pos_out = atomicAdd(&P.ctl[kHead], 1ull);
+    return ring_wait(P, pos_out, pos_out + 1);
+}
+
+__device__ __forceinline__ void ring_release(const Params &P, unsigned long long pos)
+{
+    st_release_u64(&P.pool_seq[pos & P.q_mask], pos + P.q_mask + 1);
 }
 
 // ---------------------------------------------------------------- CTA pool
@@ -752,9 +775,7 @@ __device__ bool donate_global(S &s, const Params &P)
     unsigned long long qpos = 0;
     uint32_t ok = 0;
     if (G::rank() == 0) {
-        atomicAdd(&P.ctl[kState], 1ull << 32);
         if (ring_claim_enq(P, qpos)) ok = 1;
-        else atomicAdd(&P.ctl[kState], 0xffffffff00000000ull);
     }
     ok = G::bcast(ok);
     if (!ok) { s.stat.donate_fail += 1; return false; }
@@ -770,7 +791,7 @@ __device__ bool donate_global(S &s, const Params &P)
     G::sync();
     if (G::rank() == 0) {
         __threadfence();
-        st_release_u64(&P.pool_seq[qpos & P.q_mask], qpos + 1);
+        ring_publish(P, qpos);
     }
     s.fr_bot += 1;
     s.stat.donations += 1;
@@ -1062,7 +1083,7 @@ __device__ bool acquire(S &s, const Params &P, CtaPool &cp, bool &cursor_open)
             G::sync();
             if (G::rank() == 0) {
                 __threadfence();
-                st_release_u64(&P.pool_seq[slot_i], qpos + P.q_mask + 1);
+                ring_release(P, qpos);
             }
             if (start_record<G, S>(s, P)) return true;
             if (G::rank() == 0) { __threadfence_block(); atomicAdd(&cp.hdr[kCpIdle], 1u); }

@@ -30,7 +30,8 @@ enum : uint32_t {
     kShutdown = 128,  // server: the host asks the kernel to exit once idle
     kLastWork = 144,  // server: %globaltimer of the last claimed submission
     kStarted = 160,   // server: CTAs of the launch that have started
-    kCtlWords = 176
+    kAvail = 176,     // records of the ring that are published and not yet claimed
+    kCtlWords = 192
 };
 
 enum : uint32_t { kModeMVC = 0, kModePVC = 1 };
