@@ -965,26 +965,101 @@ __device__ __forceinline__ void cover_bits(DSU<NW> &s, uint32_t *dst)
     }
 }
 
-// Stage graph `inst`'s adjacency into the CTA's bitmaps (one warp; the CTA has
-// no other active warp when this runs).
+// One warp makes row v of a graph's bitmap adjacency in `row` (NW words of its
+// own shared memory) and writes it to `out` as stage_graph copies it: kStride
+// words, chunks swizzled where the kernel's rows are.  The row's own bit, always
+// clear in a graph without self loops, carries whether v lies on a triangle.
+// Entries that break the CSR layout (a row past row_ptr[n], an id out of range, a
+// self loop) are skipped, so no read or write leaves its array; device-resident
+// input is also checked by k_check_csr, which drops a graph it flags.
 template <int NW>
-__device__ __forceinline__ void stage_graph(uint32_t *adj, const Params &P, uint32_t inst)
+__device__ __forceinline__ void prepare_row(const uint32_t *rp, const uint32_t *cl, uint32_t n, uint32_t m2, uint32_t v,
+                                            uint32_t *row, uint32_t *out)
 {
     const unsigned lane = lane_id();
-    const InstDesc d = load_desc(&P.inst[inst]);
-    const uint32_t *rp = P.row_ptr + d.row_off, *cl = P.col + d.col_off;
+    for (uint32_t w = lane; w < (uint32_t)NW; w += 32) row[w] = 0u;
+    __syncwarp();
+    const uint32_t e0 = rp[v], e1 = min(rp[v + 1], m2);
+    for (uint32_t e = e0 + lane; e < e1; e += 32) {
+        const uint32_t u = cl[e];
+        if (u < n && u != v) atomicOr(&row[u >> 5], 1u << (u & 31u));
+    }
+    __syncwarp();
+    // a neighbour of a neighbour that is a neighbour: a lane per neighbour, until one of them finds it
+    bool tri = false;
+    for (uint32_t eb = e0; eb < e1 && !tri; eb += 32) {
+        const uint32_t u = eb + lane < e1 ? cl[eb + lane] : n;
+        uint32_t f = u < n && u != v ? rp[u] : 1u;
+        const uint32_t f1 = u < n && u != v ? min(rp[u + 1], m2) : 0u;
+        while (__any_sync(0xffffffffu, f < f1)) {
+            if (f < f1) {
+                const uint32_t x = cl[f++];
+                tri = x < n && x != u && ((row[x >> 5] >> (x & 31u)) & 1u);
+            }
+            tri = __any_sync(0xffffffffu, tri);
+            if (tri) break;
+        }
+    }
+    if (lane == 0 && tri) row[v >> 5] |= 1u << (v & 31u);
+    __syncwarp();
+    for (uint32_t w = lane; w < (uint32_t)Rows<NW>::kStride; w += 32)
+        out[Rows<NW>::at(v, w)] = w < (uint32_t)NW ? row[w] : 0u;
+    __syncwarp();
+}
+
+// Stage a graph's adjacency into the CTA's bitmaps (one warp; the CTA has no
+// other active warp when this runs).  Not inlined: it is called from two rare
+// places of the search loop, which has no registers to spare for it.
+// From the rows k_prepare made: four 16-byte loads in flight per lane.
+template <int NW>
+__device__ __noinline__ void stage_rows(uint32_t *adj, const uint32_t *rows, uint32_t n)
+{
+    const unsigned lane = lane_id();
+    const uint4 *src = reinterpret_cast<const uint4 *>(rows);
+    uint4 *dst = reinterpret_cast<uint4 *>(adj);
+    const uint32_t total = (n * Rows<NW>::kStride + 3u) / 4u;
+    for (uint32_t i = lane; i < total; i += 128u) {
+        uint4 q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + 32u * k < total) q[k] = __ldcg(&src[i + 32u * k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + 32u * k < total) dst[i + 32u * k] = q[k];
+    }
+    __syncwarp();
+    for (uint32_t w = 0; w < (uint32_t)NW; ++w) {  // the rows' own bits are the tri bitmap
+        const uint32_t v = 32u * w + lane;
+        uint32_t own = 0u;
+        if (v < n) {
+            uint32_t *x = &adj[Rows<NW>::at(v, w)];
+            own = (*x >> lane) & 1u;
+            *x &= ~(1u << lane);
+        }
+        const uint32_t t = __ballot_sync(0xffffffffu, own != 0u);
+        if (lane == 0) adj[Rows<NW>::kTri + w] = t;
+    }
+    __threadfence_block();
+    __syncwarp();
+}
+
+// From the CSR, where no rows were made (servers, the allocation-free entry
+// point, batches above the bound on their memory).
+template <int NW>
+__device__ __noinline__ void stage_csr(uint32_t *adj, const uint32_t *rp, const uint32_t *cl, uint32_t n, uint32_t m2)
+{
+    const unsigned lane = lane_id();
     for (uint32_t i = lane; i < Rows<NW>::kTri + (uint32_t)NW; i += 32) adj[i] = 0;
     __syncwarp();
     // Entries that break the CSR layout (a row past row_ptr[n], an id out of
     // range, a self loop) are skipped, so no read or write leaves its array;
     // device-resident input is checked by k_check_csr before the search, which
     // drops a graph it flags.
-    const uint32_t m2 = d.m2 != kNone ? min(__ldcg(&rp[d.n]), d.m2) : __ldcg(&rp[d.n]);
-    for (uint32_t v = lane; v < d.n; v += 32) {  // row v belongs to lane v % 32
+    for (uint32_t v = lane; v < n; v += 32) {  // row v belongs to lane v % 32
         const uint32_t e1 = min(__ldcg(&rp[v + 1]), m2);
         for (uint32_t e = __ldcg(&rp[v]); e < e1; ++e) {
             const uint32_t u = __ldcg(&cl[e]);
-            if (u >= d.n || u == v) continue;
+            if (u >= n || u == v) continue;
             adj[Rows<NW>::at(v, u >> 5)] |= 1u << (u & 31u);
         }
     }
@@ -992,7 +1067,7 @@ __device__ __forceinline__ void stage_graph(uint32_t *adj, const Params &P, uint
     // tri: v has a neighbour u with a common neighbour.  Only such a vertex can
     // ever meet the triangle rule (its two live neighbours adjacent), so the
     // passes look at degree-2 vertices in tri only.
-    for (uint32_t v = lane; v < d.n; v += 32) {
+    for (uint32_t v = lane; v < n; v += 32) {
         uint32_t r[NW];
         load_row_at<NW>(adj, v, r);
         bool t = false;
@@ -1012,6 +1087,20 @@ __device__ __forceinline__ void stage_graph(uint32_t *adj, const Params &P, uint
     }
     __threadfence_block();
     __syncwarp();
+}
+
+template <int NW>
+__device__ __forceinline__ void stage_graph(uint32_t *adj, const Params &P, uint32_t inst)
+{
+    const InstDesc *d = &P.inst[inst];
+    const uint32_t n = __ldcg(&d->n);
+    if (P.adj) {
+        stage_rows<NW>(adj, P.adj + __ldcg(&d->adj_off), n);
+    } else {
+        const uint32_t *rp = P.row_ptr + __ldcg(&d->row_off);
+        const uint32_t stated = __ldcg(&d->m2), m2 = __ldcg(&rp[n]);
+        stage_csr<NW>(adj, rp, P.col + __ldcg(&d->col_off), n, stated != kNone ? min(m2, stated) : m2);
+    }
 }
 
 // Acquire work for a dense search unit.  Local records always belong to the

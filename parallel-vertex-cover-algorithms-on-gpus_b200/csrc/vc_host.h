@@ -92,7 +92,7 @@ struct Ctx {
     int coop = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    DevBuf rp, col, inst, st, covers, ctl, seq, data, gws, launches;
+    DevBuf rp, col, inst, st, covers, ctl, seq, data, gws, adj, launches;
     PinBuf h_st, h_desc, h_covers;
     unsigned long long h_ctl[vcg::kCtlWords] = {};
     bool stats_on = false;
@@ -124,6 +124,9 @@ struct Job {
     Plan plan;
 };
 
+// The most device memory a context keeps for bitmap rows (c.adj).
+constexpr uint64_t kAdjBytesMax = 4ull << 30;
+
 // The largest graph of the wide dense kernel; it also needs every degree <= 254.
 constexpr uint32_t kWideMaxN = 640;
 
@@ -152,6 +155,7 @@ struct PlanOpts {
     bool lanes = false;        // graphs <= 255 vertices take the lane kernel
     bool half = false;         // graphs of 256..1024 vertices take the 16-bit-degree dense kernels
     bool team = false;         // CSR kernels walk rows with teams of lanes (average degree >= 4)
+    bool lane = false;         // a server lane, which shares the SMs with other lanes' kernels
     const Tune *tune = nullptr; // the size class's tuned shape, if any
 };
 

@@ -220,7 +220,7 @@ extern "C" vc_status vc_solve_noalloc(const vc_csr *g, const vc_request *req, ui
     const uint32_t n = g->n;
     const int idx = n <= 64 ? 0 : (n <= 128 ? 1 : 2);
     const uint32_t nw_kernel = idx == 0 ? 2 : (idx == 1 ? 4 : 8);
-    InstDesc d;
+    InstDesc d{};
     d.n = n;
     d.nw = (n + 31) / 32;
     d.row_off = 0;

@@ -89,6 +89,7 @@ __device__ __forceinline__ InstDesc load_desc(const InstDesc *p)
     d.node_limit = __ldcg(&p->node_limit);
     d.key = __ldcg(&p->key);
     d.m2 = __ldcg(&p->m2);
+    d.adj_off = __ldcg(&p->adj_off);
     return d;
 }
 

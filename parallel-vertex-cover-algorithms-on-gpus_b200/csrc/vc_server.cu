@@ -568,12 +568,15 @@ std::vector<LaneSpec> plan_lanes(Ctx &c, uint32_t max_n)
     narrow.max_n = kDenseMax;
     narrow.per_sm = 3;
     narrow.resident = true;
-    if (make_plan(c, 32 * 8, kDenseMax, narrow.pl) != cudaSuccess || !narrow.pl.dense) return none;
+    PlanOpts no;
+    no.lane = true;
+    if (make_plan(c, 32 * 8, kDenseMax, narrow.pl, no) != cudaSuccess || !narrow.pl.dense) return none;
     wide.max_n = std::min(max_n, kWideMaxN);
     wide.per_sm = 1;
     wide.resident = true;
     PlanOpts wo;
     wo.wide = true;
+    wo.lane = true;
     if (make_plan(c, 32 * 20, kWideMaxN, wide.pl, wo) != cudaSuccess || !wide.pl.dense) return none;
     cudaFuncAttributes fw;
     if (cudaFuncGetAttributes(&fw, wide.pl.fn) != cudaSuccess) return none;
@@ -663,7 +666,9 @@ extern "C" vc_status vc_server_create(int32_t device, uint64_t mem_budget_bytes,
         s->wide_lane = true;
     } else {
         Plan pl;
-        if (make_plan(*c, std::max<uint32_t>(32, (max_n + 31) / 32 * 32), max_n, pl) != cudaSuccess) {
+        PlanOpts po;
+        po.lane = true;
+        if (make_plan(*c, std::max<uint32_t>(32, (max_n + 31) / 32 * 32), max_n, pl, po) != cudaSuccess) {
             delete s;
             return VC_ERR_CUDA;
         }

@@ -58,20 +58,18 @@ __global__ void __launch_bounds__(NT, MinThreads / NT) k_search(Params P)
     su_main<G>(P, ws, cp);
 }
 
-// Register budget of the dense search units (resident threads per SM): for
-// 8-word graphs 1280 (48 registers, five 256-thread CTAs) beat 1024 (64
-// registers) by 8% on the batched workload despite more spill traffic -- the
-// search is latency bound and more resident warps hide it; for 2/4-word graphs
-// 1536 (40 registers) measured best.
-#ifndef VC_DENSE8_THREADS
-#define VC_DENSE8_THREADS 1280
+// Register budget of the dense search units (resident threads per SM).  Graphs of
+// at most 255 vertices: 1024 (64 registers).  The packing bound keeps some twenty
+// words in registers and spills a tenth as much as with 1280 (48 registers): 1024
+// graphs of up to 200 vertices 125 -> 118 ms, one of 197 vertices 1.10 -> 1.06 ms;
+// 768 (80 registers): 121 and 0.98 ms.
+#ifndef VC_DENSE_THREADS
+#define VC_DENSE_THREADS 1024
 #endif
 #ifndef VC_DENSE_WARPS
-#define VC_DENSE_WARPS 8
+#define VC_DENSE_WARPS 4
 #endif
-#ifndef VC_DENSE4_THREADS
-#define VC_DENSE4_THREADS 1536
-#endif
+constexpr unsigned kLaneThreads = 1280;  // a server's 8-word lane: three CTAs per SM beside the other lanes' kernels
 template <int NW>
 struct DenseOcc {
     // 20-word graphs: three 256-thread CTAs' worth of registers (80 per thread),
@@ -79,13 +77,11 @@ struct DenseOcc {
     // 16- and 32-word graphs (16-bit degrees, rows and L in registers): two and
     // one CTA per SM, as many as their staged adjacency leaves room for
     static constexpr unsigned kThreads =
-        NW == 32 ? 256u : (NW == 16 ? 512u : (NW >= 16 ? 768u : (NW >= 8 ? VC_DENSE8_THREADS : VC_DENSE4_THREADS)));
-    template <unsigned NT>
-    static constexpr unsigned min_ctas() { return kThreads / NT < 32 ? kThreads / NT : 32; }  // 32 CTAs/SM at most
+        NW == 32 ? 256u : (NW == 16 ? 512u : (NW >= 16 ? 768u : VC_DENSE_THREADS));
 };
 
-template <int NW, unsigned NT>
-__global__ void __launch_bounds__(NT, DenseOcc<NW>::template min_ctas<NT>()) k_dense(Params P)
+template <int NW, unsigned NT, unsigned Threads = DenseOcc<NW>::kThreads>
+__global__ void __launch_bounds__(NT, (Threads / NT < 32 ? Threads / NT : 32)) k_dense(Params P)  // 32 CTAs/SM at most
 {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t cp_hdr[kCpHdrWords];
@@ -124,18 +120,39 @@ __global__ void __launch_bounds__(NT, 1) k_lanes(Params P)
     lanes_main<NW, NT>(P, lsm, hdr);
 }
 
-__global__ void k_init_ring(unsigned long long *seq, uint32_t q)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < q) seq[i] = i;
-}
+// What a launch needs before the search: control words, covers and counters
+// cleared, the ring's sequence numbers, the graphs' states and, for the dense
+// kernels, their adjacency as bitmap rows (A.adj; NW = 0: none), a warp per row
+// and block (x, y) the rows 32y.. of graph x.  With the rows made once by the
+// whole chip, a CTA that changes graphs copies 16-byte words instead of walking
+// CSR rows one lane per row: the first staging of a 450-vertex graph of average
+// degree 315 took over a millisecond.
+struct PrepareArgs {
+    unsigned long long *ctl, *seq;
+    uint32_t q;
+    uint32_t *covers;
+    uint32_t cover_words;
+    InstState *st;
+    const InstDesc *inst;
+    uint32_t count;
+    const uint32_t *row_ptr, *col;
+    uint32_t *adj;
+};
 
-__global__ void k_init_state(InstState *st, const InstDesc *d, uint32_t count)
+constexpr unsigned kPrepareThreads = 256;
+constexpr unsigned kPrepareRows = 32;  // per block
+
+template <int NW>
+__global__ void __launch_bounds__(kPrepareThreads) k_prepare(PrepareArgs A)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) {
+    const uint32_t block = blockIdx.x + gridDim.x * blockIdx.y;
+    const uint32_t t0 = block * kPrepareThreads + threadIdx.x, step = gridDim.x * gridDim.y * kPrepareThreads;
+    for (uint32_t i = t0; i < A.q; i += step) A.seq[i] = i;
+    for (uint32_t i = t0; i < A.cover_words; i += step) A.covers[i] = 0u;
+    for (uint32_t i = t0; i < kCtlWords; i += step) A.ctl[i] = 0ull;
+    for (uint32_t i = t0; i < A.count; i += step) {
         InstState s;
-        s.best = d[i].init_best;
+        s.best = A.inst[i].init_best;
         s.act = 1;
         s.flags = 0;
         s.lock = 0;
@@ -143,7 +160,18 @@ __global__ void k_init_state(InstState *st, const InstDesc *d, uint32_t count)
         s.pad = 0;
         s.nodes = 0;
         s.t_done = 0;
-        st[i] = s;
+        A.st[i] = s;
+    }
+    if constexpr (NW > 0) {
+        __shared__ uint32_t rows[kPrepareThreads / 32][NW];
+        for (uint32_t g = blockIdx.x; g < A.count; g += gridDim.x) {
+            const InstDesc &d = A.inst[g];
+            const uint32_t *rp = A.row_ptr + d.row_off, *cl = A.col + d.col_off;
+            const uint32_t m2 = d.m2 != kNone ? min(rp[d.n], d.m2) : rp[d.n];
+            const uint32_t lo = kPrepareRows * blockIdx.y, hi = min(d.n, lo + kPrepareRows);
+            for (uint32_t v = lo + threadIdx.x / 32; v < hi; v += kPrepareThreads / 32)
+                prepare_row<NW>(rp, cl, d.n, m2, v, rows[threadIdx.x / 32], A.adj + d.adj_off);
+        }
     }
 }
 
@@ -269,13 +297,19 @@ static uint32_t cta_pool_bytes(uint32_t slots, uint32_t stride)
 // shared memory while it fits, else in a global workspace.
 
 template <int NW>
-static cudaError_t plan_dense(Ctx &c, Plan &pl, const Tune *t)
+static cudaError_t plan_dense(Ctx &c, Plan &pl, const PlanOpts &o)
 {
+    const Tune *t = o.tune;
     pl.np = 32 * NW;
     pl.su_bytes = dense_workspace_bytes(NW);
     pl.stride = (4 + NW + 3) / 4 * 4;
     const uint32_t budget = (uint32_t)c.smem_optin - 1024;
-    uint32_t warps = (t && t->set) ? t->warps : VC_DENSE_WARPS;  // search units sharing one staged graph
+    // search units sharing one staged graph: 8, and 4 for graphs of at most 255
+    // vertices in a launch of their own, where a second copy of the rows leaves room
+    // for as many units -- a CTA can go to another graph once all its units are idle
+    // (512 graphs of 30..160 vertices 17.5 -> 15.5 ms; 2 units: 14.7, but 1024 graphs of
+    // up to 200 vertices 121 -> 125 ms)
+    uint32_t warps = (t && t->set) ? t->warps : (NW <= 8 && !o.lane ? VC_DENSE_WARPS : 8);
     const uint32_t per_warp = (t && t->set) ? t->pool : 2;
     // 32-word graphs (a 147 KB adjacency) step 8 -> 6 -> 4 warps, the others halve
     while (warps > 1 && dense_adj_bytes(NW) + warps * pl.su_bytes + cta_pool_bytes(per_warp * warps, pl.stride) > budget)
@@ -284,7 +318,14 @@ static cudaError_t plan_dense(Ctx &c, Plan &pl, const Tune *t)
     uint32_t smem = dense_adj_bytes(NW) + warps * pl.su_bytes + cta_pool_bytes(pl.cta_slots, pl.stride);
     cudaError_t e;
     switch (warps) {
-    case 8: e = plan_variant_fn<256>(c, pl, smem, k_dense<NW, 256>); break;
+    case 8:
+        if constexpr (NW == 8) {
+            e = o.lane ? plan_variant_fn<256>(c, pl, smem, k_dense<NW, 256, kLaneThreads>)
+                       : plan_variant_fn<256>(c, pl, smem, k_dense<NW, 256>);
+        } else {
+            e = plan_variant_fn<256>(c, pl, smem, k_dense<NW, 256>);
+        }
+        break;
     case 6:
         if constexpr (NW == 32) e = plan_variant_fn<192>(c, pl, smem, k_dense<NW, 192>);
         else e = cudaErrorInvalidConfiguration;
@@ -343,12 +384,12 @@ cudaError_t make_plan(Ctx &c, uint32_t np, uint32_t nmax, Plan &pl, const PlanOp
     const uint32_t smem_budget = o.smem_budget, warp_max_np = o.warp_max_np;
     // dense bitsets up to 255 vertices, and up to 640 when every degree fits a
     // byte (degrees are bytes; 0 = removed or isolated)
-    if (nmax <= 64 && !c.force_sparse) return plan_dense<2>(c, pl, o.tune);
-    if (nmax <= 128 && !c.force_sparse) return plan_dense<4>(c, pl, o.tune);
-    if (nmax <= 255 && !c.force_sparse) return plan_dense<8>(c, pl, o.tune);
-    if (nmax <= kWideMaxN && o.wide && !c.force_sparse) return plan_dense<20>(c, pl, o.tune);
+    if (nmax <= 64 && !c.force_sparse) return plan_dense<2>(c, pl, o);
+    if (nmax <= 128 && !c.force_sparse) return plan_dense<4>(c, pl, o);
+    if (nmax <= 255 && !c.force_sparse) return plan_dense<8>(c, pl, o);
+    if (nmax <= kWideMaxN && o.wide && !c.force_sparse) return plan_dense<20>(c, pl, o);
     if (nmax <= kHalfMaxN && o.half && !c.force_sparse)
-        return nmax <= 512 ? plan_dense<16>(c, pl, o.tune) : plan_dense<32>(c, pl, o.tune);
+        return nmax <= 512 ? plan_dense<16>(c, pl, o) : plan_dense<32>(c, pl, o);
     const Tune *t = (o.tune && o.tune->set && !c.force_sparse) ? o.tune : nullptr;
     pl.np = np;
     pl.su_bytes = su_workspace_bytes(np);
@@ -406,6 +447,30 @@ void cap_plan(const Ctx &c, Plan &pl, uint32_t per_sm)
     const uint32_t su_per_cta = pl.grid ? pl.num_su / pl.grid : 1;
     pl.grid = std::min(pl.grid, per_sm * (uint32_t)c.sms);
     pl.num_su = pl.grid * su_per_cta;
+}
+
+// The kernel that readies a launch (k_prepare) for bitmap rows of nw words, 0 = none.
+static cudaError_t launch_prepare(uint32_t nw, uint32_t nmax, const PrepareArgs &A, cudaStream_t stream)
+{
+    // rows: 32 per block, a column of blocks per graph; and blocks for the longest list
+    const uint32_t longest = std::max(std::max(A.q, A.cover_words), std::max<uint32_t>(A.count, kCtlWords));
+    const uint32_t lists = std::min<uint32_t>((longest + kPrepareThreads - 1) / kPrepareThreads, 64u);
+    const dim3 grid =
+        nw ? dim3(std::min<uint32_t>(A.count, 1u << 20), std::max((nmax + kPrepareRows - 1) / kPrepareRows, lists / A.count))
+           : dim3(lists);
+    const void *fn = nullptr;
+    switch (nw) {
+    case 0: fn = (const void *)k_prepare<0>; break;
+    case 2: fn = (const void *)k_prepare<2>; break;
+    case 4: fn = (const void *)k_prepare<4>; break;
+    case 8: fn = (const void *)k_prepare<8>; break;
+    case 16: fn = (const void *)k_prepare<16>; break;
+    case 20: fn = (const void *)k_prepare<20>; break;
+    case 32: fn = (const void *)k_prepare<32>; break;
+    default: return cudaErrorInvalidValue;
+    }
+    void *args[] = {const_cast<PrepareArgs *>(&A)};
+    return cudaLaunchKernel(fn, grid, dim3(kPrepareThreads), args, 0, stream);
 }
 
 // When a plain solve's units take up the packing bound (vc_dense.cuh): at once,
@@ -467,13 +532,34 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
         c.h_covers.ensure(sizeof(uint32_t) * std::max<uint32_t>(cover_words, 1)))
         return VC_ERR_NOMEM;
 
+    // bitmap rows for the dense kernels, up to a bound on what they take (above it
+    // the search units make them from the CSR when they stage a graph)
+    const uint32_t nw = pl.dense && !pl.lanes ? pl.np / 32 : 0;
+    uint64_t adj_words = 0;
+    if (nw) {
+        for (auto &d : job.desc) {
+            d.adj_off = adj_words;
+            adj_words += ((uint64_t)d.n * dense_row_words(nw) + 3) / 4 * 4;
+        }
+        if (4 * adj_words > kAdjBytesMax || c.adj.ensure(4 * adj_words)) adj_words = 0;
+    }
     memcpy(c.h_desc.p, job.desc.data(), sizeof(InstDesc) * count);
     cudaMemcpyAsync(c.inst.p, c.h_desc.p, sizeof(InstDesc) * count, cudaMemcpyHostToDevice, stream);
-    cudaMemsetAsync(c.covers.p, 0, sizeof(uint32_t) * std::max<uint32_t>(cover_words, 1), stream);
-    cudaMemsetAsync(c.ctl.p, 0, sizeof(unsigned long long) * kCtlWords, stream);
-    k_init_ring<<<(q + 255) / 256, 256, 0, stream>>>((unsigned long long *)c.seq.p, q);
-    k_init_state<<<(count + 255) / 256, 256, 0, stream>>>((InstState *)c.st.p, (const InstDesc *)c.inst.p, count);
-    g_launches += 2;
+    PrepareArgs A;
+    A.ctl = (unsigned long long *)c.ctl.p;
+    A.seq = (unsigned long long *)c.seq.p;
+    A.q = q;
+    A.covers = (uint32_t *)c.covers.p;
+    A.cover_words = cover_words;
+    A.st = (InstState *)c.st.p;
+    A.inst = (const InstDesc *)c.inst.p;
+    A.count = count;
+    A.row_ptr = job.d_rp;
+    A.col = job.d_col;
+    A.adj = adj_words ? (uint32_t *)c.adj.p : nullptr;
+    cudaEventRecord(c.ev0, stream);
+    if (launch_prepare(adj_words ? nw : 0, nmax, A, stream) != cudaSuccess) return VC_ERR_CUDA;
+    g_launches += 1;
     if (job.dev_input) {
         k_check_csr<0><<<std::min<uint32_t>(count, 4096), 256, 0, stream>>>(job.d_rp, job.d_col, (const InstDesc *)c.inst.p,
                                                                         (InstState *)c.st.p, count);
@@ -487,6 +573,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     P.inst = (const InstDesc *)c.inst.p;
     P.st = (InstState *)c.st.p;
     P.covers = (uint32_t *)c.covers.p;
+    P.adj = A.adj;
     P.count = count;
     P.num_su = pl.num_su;
     P.ctl = (unsigned long long *)c.ctl.p;
@@ -511,7 +598,6 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     P.ring_first = po.tune ? po.tune->ring_first : 0u;
 
     void *args[] = {&P};
-    cudaEventRecord(c.ev0, stream);
     cudaError_t e = c.coop ? cudaLaunchCooperativeKernel(pl.fn, dim3(pl.grid), dim3(pl.block), args, pl.smem, stream)
                            : cudaErrorNotSupported;
     if (e != cudaSuccess) return VC_ERR_CUDA;
@@ -685,7 +771,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
         job.d_rp = (const uint32_t *)c->rp.p;
         job.d_col = (const uint32_t *)c->col.p;
     }
-    InstDesc d;
+    InstDesc d{};
     d.n = g->n;
     d.nw = (g->n + 31) / 32;
     d.row_off = 0;

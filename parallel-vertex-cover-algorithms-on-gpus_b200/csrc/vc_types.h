@@ -54,6 +54,7 @@ struct InstDesc {
     uint64_t node_limit;       // 0 = none
     uint32_t key;              // unique per graph (batch index / server ticket)
     uint32_t m2;               // row_ptr[n] (2m) as the host knows it, kNone = unknown
+    uint64_t adj_off;          // word offset of this graph's bitmap rows in Params.adj
 };
 
 struct InstState {
@@ -73,6 +74,7 @@ struct Params {
     const InstDesc *inst;
     InstState *st;
     uint32_t *covers;
+    const uint32_t *adj;  // dense kernels: bitmap rows made by k_prepare, null = made from the CSR when staged
     uint32_t count;
     uint32_t num_su;
     unsigned long long *ctl;
