@@ -47,6 +47,7 @@ struct PinBuf {
     void *p = nullptr;
     size_t cap = 0;
     cudaError_t ensure(size_t bytes);
+    void release();
 };
 
 // A launch-shape choice for one size class of graphs, set by vc_autotune (or
@@ -94,6 +95,8 @@ struct Ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     DevBuf rp, col, inst, st, covers, ctl, seq, data, gws, adj, launches;
     PinBuf h_st, h_desc, h_covers;
+    DevBuf red;    // reductions of large graphs (struct Reduce)
+    PinBuf h_red;
     unsigned long long h_ctl[vcg::kCtlWords] = {};
     bool stats_on = false;
     bool force_sparse = false;
@@ -104,6 +107,28 @@ struct Ctx {
     uint32_t last_num_su = 0;
     Plan last_plan;
     std::mutex mu;
+};
+
+// What k_reduce reports of a graph (zeroed before it, but for `bad`).
+struct ReduceHead {
+    uint32_t n, m2, maxd;  // what is left: vertices, entries, largest degree
+    uint32_t taken;        // vertices taken into the cover
+    uint32_t last_pass;
+    uint32_t bad;          // the CSR check failed: nothing was reduced
+    uint32_t pad[2];
+};
+
+// A graph to reduce at its root (csrc/vc_reduce.cu) and what is left of it.
+struct Reduce {
+    const uint32_t *rp = nullptr, *cl = nullptr;  // the graph
+    uint32_t n = 0, m2 = 0, bound = 0;
+    int32_t *deg = nullptr;  // device scratch and results
+    uint32_t *taken = nullptr, *map = nullptr, *inv = nullptr, *rrp = nullptr, *rcl = nullptr, *part = nullptr;
+    uint8_t *cover = nullptr;
+    ReduceHead *head = nullptr;
+    ReduceHead h = {};                // host copies
+    const uint8_t *h_cover = nullptr;
+    uint32_t *h_inv = nullptr;
 };
 
 struct Job {
@@ -119,7 +144,8 @@ struct Job {
     bool aborted = false;
     bool wide = false;  // every graph may take the 20-word dense kernel
     bool half = false;  // every graph may take the 16/32-word dense kernels (16-bit degrees)
-    bool dev_input = false;  // the graphs came from the caller's device memory: checked by k_check_csr
+    int check = 0;  // k_check_csr before the search: 0 none, 1 the layout (caller's device memory), 2 all of it
+    std::vector<const Reduce *> rest;  // per graph: the reduction it is the rest of (empty: none are)
     const Tune *tune = nullptr;  // a shape to try instead of the context's table (the tuner's candidates)
     Plan plan;
 };
@@ -162,8 +188,10 @@ struct PlanOpts {
 Ctx *get_ctx(int dev, vc_status *err);
 cudaError_t make_plan(Ctx &c, uint32_t np, uint32_t nmax, Plan &pl, const PlanOpts &o = PlanOpts());
 void cap_plan(const Ctx &c, Plan &pl, uint32_t per_sm);
+cudaError_t launch_reduce(const Reduce &r, uint32_t ctas, cudaStream_t stream);
+uint32_t reduce_ctas(const Ctx &c);
 vc_status run_job(Ctx &c, Job &job, cudaStream_t stream);
-vc_status fill_result(const Job &job, uint32_t i, uint32_t ub, vc_result *out);
+vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_t n, vc_result *out);
 vc_status validate_csr(const vc_csr *g);
 vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_result *out, const uint32_t *d_rp,
                               const uint32_t *d_col, std::chrono::steady_clock::time_point t0);

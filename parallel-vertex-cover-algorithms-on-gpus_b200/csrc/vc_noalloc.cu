@@ -248,10 +248,10 @@ extern "C" vc_status vc_solve_noalloc(const vc_csr *g, const vc_request *req, ui
         // reads it (a graph that fails is reported VC_ERR_INVALID)
         const uint32_t *rp = g->row_ptr, *cl = g->col;
         const InstDesc *di = &s->desc;
-        InstState *sti = &s->st;
-        uint32_t one = 1;
-        void *a[] = {&rp, &cl, &di, &sti, &one};
-        if (cudaLaunchKernel((const void *)k_check_csr<0>, dim3(1), dim3(256), a, 0, stream) != cudaSuccess)
+        uint32_t *flags = &s->st.flags;
+        uint32_t stride = 1, value = kBadGraph, one = 1;
+        void *a[] = {&rp, &cl, &di, &flags, &stride, &value, &one};
+        if (cudaLaunchKernel((const void *)k_check_csr<false>, dim3(1), dim3(256), a, 0, stream) != cudaSuccess)
             return VC_ERR_CUDA;
     }
 

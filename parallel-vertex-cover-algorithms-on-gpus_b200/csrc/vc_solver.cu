@@ -211,6 +211,13 @@ cudaError_t PinBuf::ensure(size_t bytes)
     return cudaSuccess;
 }
 
+void PinBuf::release()
+{
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+}
+
 static std::mutex g_ctx_mu;
 static Ctx *g_ctx[64];
 
@@ -449,6 +456,17 @@ void cap_plan(const Ctx &c, Plan &pl, uint32_t per_sm)
     pl.num_su = pl.grid * su_per_cta;
 }
 
+// k_check_csr over `count` graphs of at most nmax vertices.
+static cudaError_t launch_check(bool full, const uint32_t *rp, const uint32_t *cl, const InstDesc *inst, uint32_t *bad,
+                                uint32_t stride, uint32_t value, uint32_t count, uint32_t nmax, cudaStream_t stream)
+{
+    const uint32_t x = std::min<uint32_t>(count, 4096);
+    const dim3 grid(x, std::max<uint32_t>(1, std::min<uint32_t>((nmax + 7) / 8, 4096 / x)));
+    void *args[] = {&rp, &cl, &inst, &bad, &stride, &value, &count};
+    return cudaLaunchKernel(full ? (const void *)k_check_csr<true> : (const void *)k_check_csr<false>, grid, dim3(256), args, 0,
+                            stream);
+}
+
 // The kernel that readies a launch (k_prepare) for bitmap rows of nw words, 0 = none.
 static cudaError_t launch_prepare(uint32_t nw, uint32_t nmax, const PrepareArgs &A, cudaStream_t stream)
 {
@@ -560,9 +578,10 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     cudaEventRecord(c.ev0, stream);
     if (launch_prepare(adj_words ? nw : 0, nmax, A, stream) != cudaSuccess) return VC_ERR_CUDA;
     g_launches += 1;
-    if (job.dev_input) {
-        k_check_csr<0><<<std::min<uint32_t>(count, 4096), 256, 0, stream>>>(job.d_rp, job.d_col, (const InstDesc *)c.inst.p,
-                                                                        (InstState *)c.st.p, count);
+    if (job.check) {
+        if (launch_check(job.check == 2, job.d_rp, job.d_col, A.inst, &A.st->flags, sizeof(InstState) / 4, kBadGraph, count,
+                         nmax, stream) != cudaSuccess)
+            return VC_ERR_CUDA;
         g_launches += 1;
     }
 
@@ -626,11 +645,41 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     return VC_OK;
 }
 
-// Fills one vc_result from the collected state of graph i.
-vc_status fill_result(const Job &job, uint32_t i, uint32_t ub, vc_result *out)
+// The bound a request's search starts from: covers smaller than this.
+static uint32_t init_best_for(const vc_request *r, uint32_t n)
+{
+    if (r->instance == VC_PVC) return n + 1;
+    uint32_t ub = r->ub ? std::min<uint32_t>(r->ub, n) : n;
+    return ub + 1;
+}
+
+// Size, decision and cover of a graph of n vertices: `found` is the size of the
+// cover found (kNone: none), `mask` writes it.
+template <class F>
+static void fill_answer(const vc_request *req, uint32_t n, uint32_t found, vc_result *out, F mask)
+{
+    if (req->instance == VC_PVC) {
+        out->decision = found != kNone ? 1u : 0u;
+        out->size = found != kNone ? found : 0u;
+    } else {
+        out->decision = 1;
+        out->size = found != kNone ? found : (req->ub ? req->ub : n);  // none below the bound: min(ub, OPT) = ub
+    }
+    out->has_cover = found != kNone ? 1u : 0u;
+    if (out->cover_mask) {
+        if (found != kNone) mask(out->cover_mask);
+        else memset(out->cover_mask, 0, n);
+    }
+}
+
+// Fills one vc_result, of a graph of n vertices, from the collected state of
+// graph i of a job: that graph, or the rest of its reduction.
+vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_t n, vc_result *out)
 {
     const InstDesc &d = job.desc[i];
     const InstState &s = job.st[i];
+    const Reduce *red = job.rest.empty() ? nullptr : job.rest[i];
+    const uint32_t taken = red ? red->h.taken : 0u;
     vc_status st;
     if (s.flags & kBadGraph) st = VC_ERR_INVALID;
     else if (s.flags & kError) st = VC_ERR_INTERNAL;
@@ -641,25 +690,127 @@ vc_status fill_result(const Job &job, uint32_t i, uint32_t ub, vc_result *out)
     out->tree_nodes = s.nodes;
     out->kernel_ms = job.kernel_ms;
     out->done_ms = (s.t_done && job.t0 && s.t_done >= job.t0) ? (float)((s.t_done - job.t0) * 1e-6) : 0.0f;
-    bool have_cover = s.cover_size != kNone;
-    if (d.mode == kModeMVC) {
-        out->decision = 1;
-        if (s.best < d.init_best) out->size = s.best;
-        else out->size = ub ? ub : d.n;  // no cover below the bound: min(ub, OPT) = ub
-    } else {
-        out->decision = (s.flags & kFound) ? 1u : 0u;
-        out->size = out->decision ? s.cover_size : 0u;
-    }
-    out->has_cover = have_cover ? 1u : 0u;
-    if (out->cover_mask) {
-        if (have_cover) {
-            const uint32_t *w = job.covers.data() + d.cover_off;
-            for (uint32_t v = 0; v < d.n; ++v) out->cover_mask[v] = (uint8_t)((w[v >> 5] >> (v & 31u)) & 1u);
+    const uint32_t found = s.cover_size != kNone ? taken + s.cover_size : kNone;
+    fill_answer(req, n, found, out, [&](uint8_t *mask) {
+        const uint32_t *w = job.covers.data() + d.cover_off;
+        if (red) {
+            memcpy(mask, red->h_cover, n);
+            for (uint32_t v = 0; v < d.n; ++v)
+                if ((w[v >> 5] >> (v & 31u)) & 1u) mask[red->h_inv[v]] = 1;
         } else {
-            memset(out->cover_mask, 0, d.n);
+            for (uint32_t v = 0; v < d.n; ++v) mask[v] = (uint8_t)((w[v >> 5] >> (v & 31u)) & 1u);
         }
-    }
+    });
     return st;
+}
+
+// ---------------------------------------------------------------- large graphs
+// Checks and reduces the graphs at their roots; the answers come back in their
+// heads and covers (one synchronisation).  `arena` says where their scratch is:
+// offsets of the rests' rows are taken from its start.
+static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, cudaStream_t stream, float *ms)
+{
+    const uint32_t count = (uint32_t)reds.size(), ctas = reduce_ctas(c);
+    size_t words = 0, host = 0;
+    auto take = [&](size_t n) {  // 16-byte pieces
+        const size_t at = words;
+        words += (n + 3) / 4 * 4;
+        return at;
+    };
+    const size_t heads = take(count * sizeof(ReduceHead) / 4), descs = take(count * sizeof(InstDesc) / 4);
+    std::vector<size_t> at;
+    for (const Reduce &r : reds) {
+        at.push_back(take(5ull * r.n + 1 + 2ull * ctas));
+        at.push_back(take(r.m2));
+        at.push_back(take((r.n + 3) / 4));
+    }
+    if (c.red.ensure(4 * words)) return VC_ERR_NOMEM;
+    uint32_t *base = (uint32_t *)c.red.p;
+    for (const Reduce &r : reds) host += (r.n + 15) / 16 * 16 + 4ull * r.n;
+    host += count * (sizeof(ReduceHead) + sizeof(InstDesc)) + 64;
+    if (c.h_red.ensure(host)) return VC_ERR_NOMEM;
+    uint8_t *h = (uint8_t *)c.h_red.p;
+    InstDesc *h_desc = (InstDesc *)h;
+    ReduceHead *h_head = (ReduceHead *)(h_desc + count);
+    uint8_t *h_at = (uint8_t *)(((uintptr_t)(h_head + count) + 15) & ~(uintptr_t)15);
+    for (uint32_t i = 0; i < count; ++i) {
+        Reduce &r = reds[i];
+        uint32_t *p = base + at[3 * i];
+        r.deg = (int32_t *)p;
+        r.taken = p + r.n;
+        r.map = p + 2ull * r.n;
+        r.inv = p + 3ull * r.n;
+        r.rrp = p + 4ull * r.n;
+        r.part = p + 5ull * r.n + 1;
+        r.rcl = base + at[3 * i + 1];
+        r.cover = (uint8_t *)(base + at[3 * i + 2]);
+        r.head = (ReduceHead *)(base + heads) + i;
+        InstDesc d{};
+        d.n = r.n;
+        d.m2 = r.m2;
+        h_desc[i] = d;
+        r.h_inv = (uint32_t *)h_at;
+        h_at += 4ull * r.n;
+        r.h_cover = h_at;
+        h_at += (r.n + 15) / 16 * 16;
+    }
+    const InstDesc *d_desc = (const InstDesc *)(base + descs);
+    bool ok = cudaMemsetAsync(base + heads, 0, count * sizeof(ReduceHead), stream) == cudaSuccess &&
+              cudaMemcpyAsync(base + descs, h_desc, count * sizeof(InstDesc), cudaMemcpyHostToDevice, stream) == cudaSuccess;
+    cudaEventRecord(c.ev0, stream);
+    for (uint32_t i = 0; ok && i < count; ++i) {
+        const Reduce &r = reds[i];
+        if (check) {
+            ok = launch_check(check == 2, r.rp, r.cl, d_desc + i, &r.head->bad, 1, 1u, 1, r.n, stream) == cudaSuccess;
+            g_launches += 1;
+        }
+        ok = ok && launch_reduce(r, ctas, stream) == cudaSuccess;
+        g_launches += 1;
+        ok = ok && cudaMemcpyAsync((void *)r.h_cover, r.cover, r.n, cudaMemcpyDeviceToHost, stream) == cudaSuccess;
+    }
+    cudaEventRecord(c.ev1, stream);
+    ok = ok && cudaMemcpyAsync(h_head, base + heads, count * sizeof(ReduceHead), cudaMemcpyDeviceToHost, stream) == cudaSuccess;
+    if (cudaStreamSynchronize(stream) != cudaSuccess || !ok) return VC_ERR_CUDA;
+    cudaEventElapsedTime(ms, c.ev0, c.ev1);
+    for (uint32_t i = 0; i < count; ++i) reds[i].h = h_head[i];
+    Plan pl;  // what vc_debug_stats reports if there is nothing left to search
+    pl.block = 512;
+    pl.grid = std::min<uint32_t>((reds.back().n + pl.block - 1) / pl.block, ctas);
+    pl.np = (reds.back().n + 31) / 32 * 32;
+    c.last_plan = pl;
+    c.last_num_su = 0;
+    c.last_stats.clear();
+    return VC_OK;
+}
+
+// The search a reduction leaves to do: false if there is none (out's answer is
+// filled in), else `d` describes the rest.
+static bool rest_of(const Reduce &r, const vc_request *req, float ms, InstDesc &d, vc_result *out)
+{
+    const uint32_t limit = req->instance == VC_PVC ? std::min<uint32_t>(req->k, r.n) : init_best_for(req, r.n) - 1;
+    if (r.h.n == 0 || r.h.taken > limit) {
+        out->status = VC_OK;
+        out->tree_nodes = 1;
+        out->kernel_ms = ms;
+        out->done_ms = ms;
+        fill_answer(req, r.n, r.h.taken <= limit ? r.h.taken : kNone, out, [&](uint8_t *m) { memcpy(m, r.h_cover, r.n); });
+        return false;
+    }
+    d.n = r.h.n;
+    d.nw = (d.n + 31) / 32;
+    d.mode = req->instance == VC_PVC ? kModePVC : kModeMVC;
+    d.k = std::min(limit - r.h.taken, d.n);
+    d.init_best = req->instance == VC_PVC ? d.n + 1 : d.k + 1;
+    d.node_limit = req->node_limit;
+    d.m2 = r.h.m2;
+    return true;
+}
+
+// A context keeps the buffers of reductions up to these sizes.
+static void trim_reductions(Ctx &c)
+{
+    if (c.red.cap > (1ull << 30)) c.red.release();
+    if (c.h_red.cap > (256ull << 20)) c.h_red.release();
 }
 
 }  // namespace vch
@@ -720,11 +871,18 @@ extern "C" uint32_t vc_debug_stats(int32_t device, int32_t enable, uint64_t *row
     return nsu;
 }
 
-static uint32_t init_best_for(const vc_request *r, uint32_t n)
+// Host-resident graphs of more entries than this are checked on the device: a
+// launch costs what the host takes for about so many.
+constexpr uint64_t kHostCheckEntries = 2048;
+
+// The checks that stay on the host when the device makes the others: what the
+// copies rely on, and the degrees, which are not copied.
+static vc_status check_head(const vc_csr *g)
 {
-    if (r->instance == VC_PVC) return n + 1;
-    uint32_t ub = r->ub ? std::min<uint32_t>(r->ub, n) : n;
-    return ub + 1;
+    if (!g->row_ptr || g->row_ptr[0] != 0 || (uint64_t)g->row_ptr[g->n] != 2ull * g->m || (g->m && !g->col)) return VC_ERR_INVALID;
+    for (uint32_t v = 0; g->degree && v < g->n; ++v)
+        if ((uint32_t)g->degree[v] != g->row_ptr[v + 1] - g->row_ptr[v]) return VC_ERR_INVALID;
+    return VC_OK;
 }
 
 extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result *out)
@@ -734,8 +892,10 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
     if (!g || !req || !out) return VC_ERR_INVALID;
     if (req->instance != VC_MVC && req->instance != VC_PVC) return VC_ERR_INVALID;
     const bool dev_in = (req->flags & VC_FLAG_DEVICE_INPUT) != 0;
-    if (!dev_in && !(req->flags & VC_FLAG_NO_VALIDATE)) {
-        vc_status v = validate_csr(g);
+    const bool validate = !dev_in && !(req->flags & VC_FLAG_NO_VALIDATE);
+    const bool on_device = validate && 2ull * g->m > kHostCheckEntries;  // the rest of the checks
+    if (validate) {
+        vc_status v = on_device ? check_head(g) : validate_csr(g);
         if (v != VC_OK) return v;
     } else if (!g->row_ptr || (g->m && !g->col)) {
         return VC_ERR_INVALID;
@@ -755,7 +915,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
     if (g->n > kMaxVertices) return VC_ERR_TOO_LARGE;
     vc_status err;
     Ctx *c = get_ctx(req->device, &err);
-    if (!c) return err;
+    if (!c) return on_device && validate_csr(g) != VC_OK ? VC_ERR_INVALID : err;
     std::lock_guard<std::mutex> lk(c->mu);
     cudaStream_t stream = req->stream ? (cudaStream_t)req->stream : c->stream;
 
@@ -771,26 +931,62 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
         job.d_rp = (const uint32_t *)c->rp.p;
         job.d_col = (const uint32_t *)c->col.p;
     }
-    InstDesc d{};
-    d.n = g->n;
-    d.nw = (g->n + 31) / 32;
-    d.row_off = 0;
-    d.col_off = 0;
-    d.mode = req->instance == VC_PVC ? kModePVC : kModeMVC;
-    d.k = std::min<uint32_t>(req->k, g->n);
-    d.init_best = init_best_for(req, g->n);
-    d.cover_off = 0;
-    d.node_limit = req->node_limit;
-    d.key = 0;
-    d.m2 = 2ull * g->m < (uint64_t)kNone ? (uint32_t)(2ull * g->m) : kNone;
-    job.desc.push_back(d);
+    job.check = dev_in ? 1 : (on_device ? 2 : 0);
     job.time_limit_s = req->time_limit_s;
-    job.wide = !dev_in && wide_ok(g->n, g->row_ptr);
-    job.half = !job.wide && half_ok(g->n);
-    job.dev_input = dev_in;
+    InstDesc d{};
+    float reduce_ms = 0;
+    std::vector<Reduce> red;
+    if (g->n > kHalfMaxN && !c->force_sparse && 2ull * g->m < kNone) {
+        // a large graph: its root is reduced by the whole chip, the search gets the rest
+        Reduce r;
+        r.rp = job.d_rp;
+        r.cl = job.d_col;
+        r.n = g->n;
+        r.m2 = 2 * g->m;
+        r.bound = req->instance == VC_PVC ? std::min<uint32_t>(req->k, g->n) + 1 : init_best_for(req, g->n);
+        red.push_back(r);
+        const vc_status s = run_reductions(*c, red, job.check, stream, &reduce_ms);
+        if (s == VC_ERR_NOMEM) {
+            red.clear();  // no room for it: the search reduces the root itself
+        } else {
+            const bool bad = s == VC_OK && red[0].h.bad;
+            if (s != VC_OK || bad) {
+                out->status = bad ? VC_ERR_INVALID : s;
+                trim_reductions(*c);
+                return out->status;
+            }
+            if (!rest_of(red[0], req, reduce_ms, d, out)) {
+                trim_reductions(*c);
+                out->total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+                return VC_OK;
+            }
+            job.d_rp = red[0].rrp;
+            job.d_col = red[0].rcl;
+            job.check = 0;
+            job.rest.push_back(&red[0]);
+            cudaMemcpyAsync(red[0].h_inv, red[0].inv, 4ull * d.n, cudaMemcpyDeviceToHost, stream);
+            job.wide = d.n <= kWideMaxN && red[0].h.maxd <= 254;
+        }
+    }
+    if (red.empty()) {
+        d.n = g->n;
+        d.nw = (g->n + 31) / 32;
+        d.mode = req->instance == VC_PVC ? kModePVC : kModeMVC;
+        d.k = std::min<uint32_t>(req->k, g->n);
+        d.init_best = init_best_for(req, g->n);
+        d.node_limit = req->node_limit;
+        d.m2 = 2ull * g->m < (uint64_t)kNone ? (uint32_t)(2ull * g->m) : kNone;
+        job.wide = !dev_in && wide_ok(g->n, g->row_ptr);
+    }
+    job.half = !job.wide && half_ok(d.n);
+    job.desc.push_back(d);
     vc_status s = run_job(*c, job, stream);
+    if (s == VC_OK && (job.st[0].flags & kBadGraph)) s = VC_ERR_INVALID;
     if (s != VC_OK) { out->status = s; return s; }
-    s = fill_result(job, 0, req->instance == VC_MVC ? req->ub : 0, out);
+    s = fill_result(job, 0, req, g->n, out);
+    out->kernel_ms += reduce_ms;
+    out->done_ms += reduce_ms;
+    trim_reductions(*c);
     out->total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return s;
 }
@@ -835,22 +1031,29 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         const uint32_t *rp = a->row_ptr + a->row_off[i];
         cols = std::max<uint64_t>(cols, a->col_off[i] + rp[a->n[i]]);
     }
-    if (!d_rp && !(reqs[0].flags & VC_FLAG_NO_VALIDATE)) {
+    const bool validate = !d_rp && !(reqs[0].flags & VC_FLAG_NO_VALIDATE);
+    const bool on_device = validate && cols > kHostCheckEntries;
+    auto host_checks = [&](bool all) {
         for (uint32_t i = 0; i < count; ++i) {
             vc_csr g;
             g.n = a->n[i];
             const uint32_t *rp = a->row_ptr + a->row_off[i];
             g.m = rp[g.n] / 2;
             g.row_ptr = rp;
-            g.col = a->col + a->col_off[i];
+            g.col = a->col ? a->col + a->col_off[i] : nullptr;
             g.degree = nullptr;
-            vc_status v = validate_csr(&g);
-            if (v != VC_OK) return fail(v);
+            const vc_status v = all ? validate_csr(&g) : check_head(&g);
+            if (v != VC_OK) return v;
         }
+        return VC_OK;
+    };
+    if (validate) {
+        const vc_status v = host_checks(!on_device);
+        if (v != VC_OK) return fail(v);
     }
     vc_status err;
     Ctx *c = get_ctx(reqs[0].device, &err);
-    if (!c) return fail(err);
+    if (!c) return fail(on_device && host_checks(true) != VC_OK ? VC_ERR_INVALID : err);
     std::lock_guard<std::mutex> lk(c->mu);
     cudaStream_t stream = reqs[0].stream ? (cudaStream_t)reqs[0].stream : c->stream;
     Job job;
@@ -865,63 +1068,154 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         job.d_rp = (const uint32_t *)c->rp.p;
         job.d_col = (const uint32_t *)c->col.p;
     }
+    const int check = d_rp ? 1 : (on_device ? 2 : 0);
+    float total_kernel = 0;
+    // Large graphs first: each root is reduced by the whole chip, and the search
+    // gets what is left of it.
+    std::vector<Reduce> reds;
+    std::vector<uint32_t> red_of;  // the graph each reduction is of
+    if (!c->force_sparse) {
+        for (uint32_t i = 0; i < count; ++i) {
+            if (a->n[i] <= kHalfMaxN) continue;
+            const uint32_t *rp = a->row_ptr + a->row_off[i];
+            Reduce r;
+            r.rp = job.d_rp + a->row_off[i];
+            r.cl = job.d_col + a->col_off[i];
+            r.n = a->n[i];
+            r.m2 = rp[r.n];
+            r.bound = reqs[i].instance == VC_PVC ? std::min<uint32_t>(reqs[i].k, r.n) + 1 : init_best_for(&reqs[i], r.n);
+            reds.push_back(r);
+            red_of.push_back(i);
+        }
+    }
+    struct Trim {
+        Ctx *c;
+        ~Trim() { trim_reductions(*c); }
+    } trim{c};
+    if (!reds.empty()) {
+        const vc_status s = run_reductions(*c, reds, check, stream, &total_kernel);
+        if (s == VC_ERR_NOMEM) {
+            reds.clear();  // no room: the search reduces the roots itself
+            red_of.clear();
+        } else if (s != VC_OK) {
+            return fail(s);
+        }
+    }
+    std::vector<const Reduce *> red_at(count, nullptr);
+    for (size_t j = 0; j < reds.size(); ++j) red_at[red_of[j]] = &reds[j];
+    if (check == 2)
+        for (const Reduce &r : reds)
+            if (r.h.bad) return fail(VC_ERR_INVALID);
+    vc_status first = VC_OK;
+    std::vector<vc_status> got(count, VC_OK);
     // One launch per kernel shape: dense bitsets (n <= 255), wide dense bitsets
     // (n <= 640, every degree <= 254), dense bitsets with 16-bit degrees (n <=
     // 1024), warp search units (n <= kWarpMaxNP), CTA search units (larger); the
     // shape is sized by the largest graph of its class, so small graphs never
     // run in a large graph's workspace.  The row offsets are host arrays on both
-    // entry points.
-    auto klass = [&](uint32_t i) {
-        const uint32_t n = a->n[i];
+    // entry points.  The rests of reductions are classes 5 to 9, in launches of
+    // their own: their rows are not in the arena.
+    auto klass = [&](uint32_t n, bool wide) {
         if (n <= 255) return 0;
-        if (wide_ok(n, a->row_ptr + a->row_off[i])) return 1;
+        if (wide) return 1;
         if (half_ok(n)) return 2;
         return n <= kWarpMaxNP ? 3 : 4;
     };
-    vc_status first = VC_OK;
-    float total_kernel = 0;
-    std::vector<uint32_t> members;
-    for (int cl = 0; cl < 5; ++cl) {
-        members.clear();
+    std::vector<int> cls(count, -1);
+    std::vector<InstDesc> rest(reds.size());
+    std::vector<vc_result> early(reds.size());  // answers of graphs without a rest
+    std::vector<uint8_t> searched(reds.size(), 0);
+    for (size_t j = 0; j < reds.size(); ++j) {
+        const uint32_t i = red_of[j];
+        Reduce &r = reds[j];
+        early[j] = out[i];
+        if (r.h.bad) {  // device-resident input: this graph only
+            early[j].cover_mask = nullptr;
+            fill_answer(&reqs[i], r.n, kNone, &early[j], [](uint8_t *) {});
+            early[j].status = VC_ERR_INVALID;
+            early[j].tree_nodes = 0;
+            early[j].done_ms = 0;
+            continue;
+        }
+        rest[j] = InstDesc{};
+        early[j].cover_mask = nullptr;  // written below, when every launch has gone well
+        if (!rest_of(r, &reqs[i], total_kernel, rest[j], &early[j])) continue;
+        searched[j] = 1;
+        cudaMemcpyAsync(r.h_inv, r.inv, 4ull * rest[j].n, cudaMemcpyDeviceToHost, stream);
+        cls[i] = 5 + klass(rest[j].n, rest[j].n <= kWideMaxN && r.h.maxd <= 254);
+    }
+    for (uint32_t i = 0; i < count; ++i)
+        if (a->n[i] > 0 && !red_at[i]) cls[i] = klass(a->n[i], wide_ok(a->n[i], a->row_ptr + a->row_off[i]));
+    std::vector<Job> jobs;
+    std::vector<std::vector<uint32_t>> members;
+    for (int cl = 0; cl < 10; ++cl) {
+        std::vector<uint32_t> mem;
         for (uint32_t i = 0; i < count; ++i)
-            if (a->n[i] > 0 && klass(i) == cl) members.push_back(i);
-        if (members.empty()) continue;
+            if (cls[i] == cl) mem.push_back(i);
+        if (mem.empty()) continue;
         Job cj;
-        cj.d_rp = job.d_rp;
-        cj.d_col = job.d_col;
-        cj.wide = cl == 1;
-        cj.half = cl == 2;
-        cj.dev_input = d_rp != nullptr;
-        cj.desc.resize(members.size());
+        const bool rests = cl >= 5;
+        cj.d_rp = rests ? (const uint32_t *)c->red.p : job.d_rp;
+        cj.d_col = rests ? (const uint32_t *)c->red.p : job.d_col;
+        cj.wide = cl % 5 == 1;
+        cj.half = cl % 5 == 2;
+        cj.check = rests ? 0 : check;
+        cj.desc.resize(mem.size());
         double tl = 0;
-        for (size_t j = 0; j < members.size(); ++j) {
-            const uint32_t i = members[j];
+        for (size_t j = 0; j < mem.size(); ++j) {
+            const uint32_t i = mem[j];
             InstDesc &d = cj.desc[j];
-            d.n = a->n[i];
-            d.nw = (d.n + 31) / 32;
-            d.row_off = a->row_off[i];
-            d.col_off = a->col_off[i];
-            d.mode = reqs[i].instance == VC_PVC ? kModePVC : kModeMVC;
-            d.k = std::min<uint32_t>(reqs[i].k, d.n);
-            d.init_best = init_best_for(&reqs[i], d.n);
-            d.node_limit = reqs[i].node_limit;
+            if (rests) {
+                const Reduce *r = red_at[i];
+                d = rest[r - reds.data()];
+                d.row_off = (uint64_t)(r->rrp - (const uint32_t *)c->red.p);
+                d.col_off = (uint64_t)(r->rcl - (const uint32_t *)c->red.p);
+                cj.rest.push_back(r);
+            } else {
+                d.n = a->n[i];
+                d.nw = (d.n + 31) / 32;
+                d.row_off = a->row_off[i];
+                d.col_off = a->col_off[i];
+                d.mode = reqs[i].instance == VC_PVC ? kModePVC : kModeMVC;
+                d.k = std::min<uint32_t>(reqs[i].k, d.n);
+                d.init_best = init_best_for(&reqs[i], d.n);
+                d.node_limit = reqs[i].node_limit;
+                d.m2 = a->row_ptr[a->row_off[i] + d.n];
+            }
             d.key = (uint32_t)j;
-            d.m2 = a->row_ptr[a->row_off[i] + d.n];
             tl = std::max(tl, reqs[i].time_limit_s);
         }
         cj.time_limit_s = tl;
         vc_status s = run_job(*c, cj, stream);
+        if (s == VC_OK && check == 2)
+            for (const InstState &st : cj.st)
+                if (st.flags & kBadGraph) return fail(VC_ERR_INVALID);
         if (s != VC_OK) {
             for (uint32_t i = 0; i < count; ++i) out[i].status = s;
             return s;
         }
         total_kernel += cj.kernel_ms;
-        for (size_t j = 0; j < members.size(); ++j) {
-            const uint32_t i = members[j];
-            vc_status si = fill_result(cj, (uint32_t)j, reqs[i].instance == VC_MVC ? reqs[i].ub : 0, &out[i]);
-            if (si != VC_OK && first == VC_OK) first = si;
-        }
+        jobs.push_back(std::move(cj));
+        members.push_back(std::move(mem));
     }
+    for (size_t q = 0; q < jobs.size(); ++q)
+        for (size_t j = 0; j < members[q].size(); ++j) {
+            const uint32_t i = members[q][j];
+            got[i] = fill_result(jobs[q], (uint32_t)j, &reqs[i], a->n[i], &out[i]);
+        }
+    for (size_t j = 0; j < reds.size(); ++j) {
+        if (searched[j]) continue;
+        const uint32_t i = red_of[j];
+        uint8_t *mask = out[i].cover_mask;
+        out[i] = early[j];
+        out[i].cover_mask = mask;
+        if (mask) {
+            if (out[i].has_cover) memcpy(mask, reds[j].h_cover, reds[j].n);
+            else memset(mask, 0, reds[j].n);
+        }
+        got[i] = out[i].status;
+    }
+    for (uint32_t i = 0; i < count && first == VC_OK; ++i) first = got[i];
     float total = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     for (uint32_t i = 0; i < count; ++i) {
         out[i].total_ms = total;
