@@ -17,6 +17,16 @@ static bool row_has(const uint32_t *rp, const uint32_t *col, uint32_t row, uint3
     return std::binary_search(b, e, x);
 }
 
+// The checks that stay on the host when the device makes the others: what the
+// copies rely on, and the degrees, which are not copied.
+vc_status check_head(const vc_csr *g)
+{
+    if (!g->row_ptr || g->row_ptr[0] != 0 || (uint64_t)g->row_ptr[g->n] != 2ull * g->m || (g->m && !g->col)) return VC_ERR_INVALID;
+    for (uint32_t v = 0; g->degree && v < g->n; ++v)
+        if ((uint32_t)g->degree[v] != g->row_ptr[v + 1] - g->row_ptr[v]) return VC_ERR_INVALID;
+    return VC_OK;
+}
+
 vc_status validate_csr(const vc_csr *g)
 {
     if (!g->row_ptr) return VC_ERR_INVALID;

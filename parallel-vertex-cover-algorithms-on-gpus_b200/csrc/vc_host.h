@@ -95,6 +95,7 @@ struct Ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     DevBuf rp, col, inst, st, covers, ctl, seq, data, gws, adj, launches;
     PinBuf h_st, h_desc, h_covers;
+    DevBuf ub;     // the upper-bound heuristics (vc_ub.cu)
     DevBuf red;    // reductions of large graphs (struct Reduce)
     PinBuf h_red;
     unsigned long long h_ctl[vcg::kCtlWords] = {};
@@ -153,6 +154,9 @@ struct Job {
 // The most device memory a context keeps for bitmap rows (c.adj).
 constexpr uint64_t kAdjBytesMax = 4ull << 30;
 
+// The most device memory a context keeps for the upper-bound heuristics (c.ub).
+constexpr uint64_t kUbBytesKept = 1ull << 30;
+
 // The largest graph of the wide dense kernel; it also needs every degree <= 254.
 constexpr uint32_t kWideMaxN = 640;
 
@@ -193,6 +197,10 @@ uint32_t reduce_ctas(const Ctx &c);
 vc_status run_job(Ctx &c, Job &job, cudaStream_t stream);
 vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_t n, vc_result *out);
 vc_status validate_csr(const vc_csr *g);
+vc_status check_head(const vc_csr *g);
+cudaError_t launch_check(bool full, const uint32_t *rp, const uint32_t *cl, const vcg::InstDesc *inst, uint32_t *bad,
+                         uint32_t stride, uint32_t value, uint32_t count, uint32_t nmax, cudaStream_t stream,
+                         uint32_t *mate = nullptr);
 vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_result *out, const uint32_t *d_rp,
                               const uint32_t *d_col, std::chrono::steady_clock::time_point t0);
 

@@ -249,8 +249,8 @@ extern "C" vc_status vc_solve_noalloc(const vc_csr *g, const vc_request *req, ui
         const uint32_t *rp = g->row_ptr, *cl = g->col;
         const InstDesc *di = &s->desc;
         uint32_t *flags = &s->st.flags;
-        uint32_t stride = 1, value = kBadGraph, one = 1;
-        void *a[] = {&rp, &cl, &di, &flags, &stride, &value, &one};
+        uint32_t stride = 1, value = kBadGraph, one = 1, *mate = nullptr;
+        void *a[] = {&rp, &cl, &di, &flags, &stride, &value, &one, &mate};
         if (cudaLaunchKernel((const void *)k_check_csr<false>, dim3(1), dim3(256), a, 0, stream) != cudaSuccess)
             return VC_ERR_CUDA;
     }

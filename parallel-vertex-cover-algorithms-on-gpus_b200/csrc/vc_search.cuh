@@ -102,8 +102,11 @@ __device__ __forceinline__ InstDesc load_desc(const InstDesc *p)
 // word of `bad`.  Full is the host's check (vc_host.cpp) where that is the slower:
 // a graph of 100,000 vertices and 383,000 edges takes the host 27 ms, one of 450 and
 // 71,000 2.3 ms; here the dependent loads of one binary search, some 10 us.
+// `mate` (Full, may be null) receives for every entry the place of the edge's other
+// entry.
 template <bool Full>
-__device__ __forceinline__ bool check_row(const uint32_t *rp, const uint32_t *cl, uint32_t n, uint32_t m2, uint32_t v)
+__device__ __forceinline__ bool check_row(const uint32_t *rp, const uint32_t *cl, uint32_t n, uint32_t m2, uint32_t v,
+                                          uint32_t *mate)
 {
     const uint32_t e0 = rp[v], e1 = rp[v + 1];
     if (e1 < e0 || e1 > m2) return true;
@@ -119,6 +122,7 @@ __device__ __forceinline__ bool check_row(const uint32_t *rp, const uint32_t *cl
             while (lo < hi && !found) {
                 const uint32_t mid = lo + (hi - lo) / 2, c = cl[mid];
                 found = c == v;
+                if (found && mate) mate[e] = mid;
                 if (c < v) lo = mid + 1; else hi = mid;
             }
             bad |= !found;
@@ -129,7 +133,8 @@ __device__ __forceinline__ bool check_row(const uint32_t *rp, const uint32_t *cl
 
 template <bool Full>
 __global__ void __launch_bounds__(256) k_check_csr(const uint32_t *row_ptr, const uint32_t *col, const InstDesc *inst,
-                                                   uint32_t *bad, uint32_t bad_stride, uint32_t value, uint32_t count)
+                                                   uint32_t *bad, uint32_t bad_stride, uint32_t value, uint32_t count,
+                                                   uint32_t *mate)
 {
     for (uint32_t gi = blockIdx.x; gi < count; gi += gridDim.x) {
         const InstDesc &d = inst[gi];
@@ -138,7 +143,7 @@ __global__ void __launch_bounds__(256) k_check_csr(const uint32_t *row_ptr, cons
         bool b = rp[0] != 0u || (d.m2 != kNone && m2 != d.m2);
         if (!b)
             for (uint32_t v = 8u * blockIdx.y + (threadIdx.x >> 5); v < d.n; v += 8u * gridDim.y)
-                b |= check_row<Full>(rp, cl, d.n, m2, v);
+                b |= check_row<Full>(rp, cl, d.n, m2, v, mate ? mate + d.col_off : nullptr);
         if (__syncthreads_or(b) && threadIdx.x == 0) atomicOr(&bad[(size_t)gi * bad_stride], value);
     }
 }

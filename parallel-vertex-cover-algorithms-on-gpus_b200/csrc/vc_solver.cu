@@ -457,12 +457,12 @@ void cap_plan(const Ctx &c, Plan &pl, uint32_t per_sm)
 }
 
 // k_check_csr over `count` graphs of at most nmax vertices.
-static cudaError_t launch_check(bool full, const uint32_t *rp, const uint32_t *cl, const InstDesc *inst, uint32_t *bad,
-                                uint32_t stride, uint32_t value, uint32_t count, uint32_t nmax, cudaStream_t stream)
+cudaError_t launch_check(bool full, const uint32_t *rp, const uint32_t *cl, const InstDesc *inst, uint32_t *bad,
+                                uint32_t stride, uint32_t value, uint32_t count, uint32_t nmax, cudaStream_t stream, uint32_t *mate)
 {
     const uint32_t x = std::min<uint32_t>(count, 4096);
     const dim3 grid(x, std::max<uint32_t>(1, std::min<uint32_t>((nmax + 7) / 8, 4096 / x)));
-    void *args[] = {&rp, &cl, &inst, &bad, &stride, &value, &count};
+    void *args[] = {&rp, &cl, &inst, &bad, &stride, &value, &count, &mate};
     return cudaLaunchKernel(full ? (const void *)k_check_csr<true> : (const void *)k_check_csr<false>, grid, dim3(256), args, 0,
                             stream);
 }
@@ -874,16 +874,6 @@ extern "C" uint32_t vc_debug_stats(int32_t device, int32_t enable, uint64_t *row
 // Host-resident graphs of more entries than this are checked on the device: a
 // launch costs what the host takes for about so many.
 constexpr uint64_t kHostCheckEntries = 2048;
-
-// The checks that stay on the host when the device makes the others: what the
-// copies rely on, and the degrees, which are not copied.
-static vc_status check_head(const vc_csr *g)
-{
-    if (!g->row_ptr || g->row_ptr[0] != 0 || (uint64_t)g->row_ptr[g->n] != 2ull * g->m || (g->m && !g->col)) return VC_ERR_INVALID;
-    for (uint32_t v = 0; g->degree && v < g->n; ++v)
-        if ((uint32_t)g->degree[v] != g->row_ptr[v + 1] - g->row_ptr[v]) return VC_ERR_INVALID;
-    return VC_OK;
-}
 
 extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result *out)
 {
