@@ -365,11 +365,11 @@ __device__ __forceinline__ uint32_t pack_pick(const uint32_t *adj, uint32_t e, u
                                               uint32_t &picked)
 {
     using PG = PackGroup<NW>;
+    // the lowest vertex of each word, found while the ballot is under way
+    const uint32_t bit = e & (0u - e), low = 32u * word + (31u - __clz(bit | 1u));
     const uint32_t src = bal ? __ffs(bal) - 1 : 0u;  // the word it is in
-    const uint32_t bit = word == src ? e & (0u - e) : 0u;
-    picked |= bit;
-    const uint32_t at = PG::kGroups == 1 ? src : src + (lane_id() & 16u);
-    const uint32_t v = 32u * src + (31u - __clz(__shfl_sync(0xffffffffu, bit, at) | 1u));
+    if (word == src) picked |= bit;
+    const uint32_t v = __shfl_sync(0xffffffffu, low, PG::kGroups == 1 ? src : src + (lane_id() & 16u));
     return adj[Rows<NW>::at(v, word < (uint32_t)NW ? word : 0u)] & live;
 }
 
@@ -1103,6 +1103,120 @@ __device__ __forceinline__ void stage_graph(uint32_t *adj, const Params &P, uint
     }
 }
 
+// ---- first covers
+// A plain solve of a graph of 16 words or more whose average degree is at most 16
+// starts with dives on the first blocks after the one that takes up the search: the
+// last 913-vertex graph of a sparse pair went from 1.9 to 1.0 ms with its partner,
+// four graphs of 327..584 vertices from 4.6 to 3.5.  Dense graphs gain nothing; and
+// with smaller ones the nodes fall as much (175 vertices: 6,700 to 530) but not the
+// time (0.39 to 0.59 ms): against a tight incumbent a node's bound runs its full
+// course, and the chain of nodes to the first leaf is what such a tree's time is.
+constexpr uint32_t kDiveBlocks = 37;
+// One greedy dive: a vertex of least degree, at random among them, stays out of
+// the cover and its neighbours go in, until no edge is left.  The cover is left in
+// `cover` (NW words) and its size returned; a dive that reaches `limit` vertices
+// gives up.  Search units that would wait for work make a dive each: on sparse random
+// graphs the best of a hundred is usually a minimum cover, and a search that prunes
+// against it from the start opens a third to a tenth of the nodes that it opens
+// while its own first leaves come in.
+template <int NW>
+__device__ __noinline__ uint32_t dense_dive(const uint32_t *adj, uint32_t *cover, uint32_t n, uint32_t limit, uint32_t seed)
+{
+    constexpr int K = Rows<NW>::kHalf ? 10 : 8;  // planes: every degree of the kernel's graphs
+    const unsigned lane = lane_id();
+    const uint32_t at = lane < (uint32_t)NW ? lane : 0u;
+    uint32_t B[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) B[k] = 0u;
+    for (uint32_t w = 0; 32u * w < n; ++w) {
+        const uint32_t v = 32u * w + lane;
+        uint32_t d = 0;
+        if (v < n) {
+            uint32_t r[NW];
+            load_row_at<NW>(adj, v, r);
+#pragma unroll
+            for (int i = 0; i < NW; ++i) d += __popc(r[i]);
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t x = __ballot_sync(0xffffffffu, (d >> k) & 1u);
+            if (lane == w) B[k] = x;
+        }
+    }
+    uint32_t live = 0u, cov = 0u, size = 0u;
+#pragma unroll
+    for (int k = 0; k < K; ++k) live |= B[k];
+    for (uint32_t it = 0; it < n; ++it) {
+        uint32_t c = live;  // the vertices of least degree
+#pragma unroll
+        for (int k = K - 1; k >= 0; --k) {
+            const uint32_t t = c & ~B[k];
+            if (__any_sync(0xffffffffu, t != 0u)) c = t;
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, c != 0u);
+        if (!bal) break;
+        seed = seed * 1664525u + 1013904223u;
+        const uint32_t r1 = seed >> 27, r2 = (seed >> 22) & 31u;
+        const uint32_t src = (__ffs(__funnelshift_r(bal, bal, r1)) - 1 + r1) & 31u;
+        c = __shfl_sync(0xffffffffu, c, src);
+        const uint32_t b = (__ffs(__funnelshift_r(c, c, r2)) - 1 + r2) & 31u;
+        const uint32_t nb = adj[Rows<NW>::at(32u * src + b, at)] & live;
+        cov |= nb;
+        size += __reduce_add_sync(0xffffffffu, __popc(nb));
+        if (size >= limit) return size;
+        uint32_t wm = __ballot_sync(0xffffffffu, nb != 0u);
+        while (wm) {
+            const uint32_t w = __ffs(wm) - 1;
+            wm &= wm - 1;
+            uint32_t m = __shfl_sync(0xffffffffu, nb, w);
+            while (m) {
+                const uint32_t u = 32u * w + (__ffs(m) - 1);
+                m &= m - 1;
+                uint32_t br = adj[Rows<NW>::at(u, at)] & live;
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const uint32_t t = B[k];
+                    B[k] = t ^ br;
+                    br &= ~t;
+                }
+            }
+        }
+        const uint32_t gone = nb | (lane == src ? 1u << b : 0u);
+        live = 0u;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            B[k] &= ~gone;
+            live |= B[k];
+        }
+    }
+    if (lane < (uint32_t)NW) cover[lane] = cov;
+    __syncwarp();
+    return size;
+}
+
+// A dive on the CTA's staged graph `inst` by a unit without work; a cover that
+// betters the incumbent (PVC: answers the question) is reported.  The unit holds no
+// token of the graph: its CTA is not idle meanwhile, so the launch outlasts it.
+template <int NW>
+__device__ __forceinline__ void dive_on(DSU<NW> &s, const Params &P, uint32_t inst)
+{
+    using S = DSU<NW>;
+    const unsigned lane = lane_id();
+    const uint32_t n = __ldcg(&P.inst[inst].n), mode = __ldcg(&P.inst[inst].mode);
+    const uint32_t limit = mode == kModePVC ? __ldcg(&P.inst[inst].k) + 1u
+                                            : WarpG::bcast(ld_relaxed_u32(&P.st[inst].best));
+    const uint32_t size = dense_dive<NW>(s.adj, s.bits(), n, limit, 2654435761u * (WarpG::su_global() + 1u) + inst);
+    if (size >= limit) return;
+    if (lane < NW) {
+        const uint32_t lo = 32u * lane;
+        s.lsm()[lane] = ~s.bits()[lane] & (lo + 32u <= n ? 0xffffffffu : (lo < n ? (1u << (n - lo)) - 1u : 0u));
+    }
+    __syncwarp();
+    bind_graph<WarpG>(s, P, inst);
+    report_leaf<WarpG, S>(s, P, size);
+    s.inst = kNone;
+}
+
 // Acquire work for a dense search unit.  Local records always belong to the
 // CTA's staged graph.  Only when the whole CTA is idle may the poller switch
 // graphs: first to the next root from the cursor, then to records of any graph
@@ -1250,7 +1364,8 @@ __device__ bool acquire_cta(DSU<NW> &s, const Params &P, CtaPool &cp, uint32_t *
             continue;
         }
         if (lane == 0) __nanosleep(nap);
-        nap = nap < (poller ? 4096u : kIdleNapMax) ? nap * 2 : (poller ? 4096u : kIdleNapMax);
+        const uint32_t most = P.count == 1 ? kPlainNapMax : (poller ? 4096u : kIdleNapMax);
+        nap = nap < most ? nap * 2 : most;
         __syncwarp();
     }
 }
@@ -1286,6 +1401,14 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
     const uint32_t tick_mask = P.count == 1 ? 1u : 7u;
     bool packing = P.pack_after_ns == 0;
     const unsigned long long t_pack = globaltimer() + P.pack_after_ns;
+    if (NW >= 16 && P.dives && blockIdx.x - 1u < kDiveBlocks) {  // block 0 takes up the search
+        if (WarpG::su_local() == 0) {
+            stage_graph<NW>(adj, P, 0);
+            if (lane == 0) cp.hdr[kCpStaged] = __ldcg(&P.inst[0].key);
+        }
+        __syncthreads();
+        if (!(G::bcast(ld_relaxed_u32(&P.st[0].flags)) & kBadGraph)) dive_on<NW>(s, P, 0);
+    }
 
     for (;;) {
         if (!have) {

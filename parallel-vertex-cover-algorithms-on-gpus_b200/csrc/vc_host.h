@@ -185,6 +185,7 @@ struct PlanOpts {
     bool lanes = false;        // graphs <= 255 vertices take the lane kernel
     bool half = false;         // graphs of 256..1024 vertices take the 16-bit-degree dense kernels
     bool team = false;         // CSR kernels walk rows with teams of lanes (average degree >= 4)
+    bool plain = false;        // a launch of one graph
     bool lane = false;         // a server lane, which shares the SMs with other lanes' kernels
     const Tune *tune = nullptr; // the size class's tuned shape, if any
 };

@@ -157,6 +157,10 @@ __global__ void __launch_bounds__(256) k_check_csr(const uint32_t *row_ptr, cons
 #define VC_IDLE_NAP_MAX 16384u
 #endif
 constexpr uint32_t kIdleNapMax = VC_IDLE_NAP_MAX;
+// A plain solve's units nap this long at most: small trees end sooner by a nap or
+// two (path of 60 vertices 85 -> 57 us, G(60, 0.1) 148 -> 129); a batch loses by it
+// (1024 graphs 120 -> 125 ms).
+constexpr uint32_t kPlainNapMax = 2048u;
 
 // ---------------------------------------------------------------- groups
 struct WarpG {

@@ -61,14 +61,17 @@ __global__ void __launch_bounds__(NT, MinThreads / NT) k_search(Params P)
 // Register budget of the dense search units (resident threads per SM).  Graphs of
 // at most 255 vertices: 1024 (64 registers).  The packing bound keeps some twenty
 // words in registers and spills a tenth as much as with 1280 (48 registers): 1024
-// graphs of up to 200 vertices 125 -> 118 ms, one of 197 vertices 1.10 -> 1.06 ms;
-// 768 (80 registers): 121 and 0.98 ms.
+// graphs of up to 200 vertices 125 -> 118 ms; 768 (80 registers): 121, 512: 130.  A
+// plain solve has idle units and waits for its longest chain of nodes: 512 (128
+// registers, no spills), eight calls on G(60, 0.1) 1.07 -> 0.91 ms, one of 197
+// vertices 0.99 -> 0.84.
 #ifndef VC_DENSE_THREADS
 #define VC_DENSE_THREADS 1024
 #endif
 #ifndef VC_DENSE_WARPS
 #define VC_DENSE_WARPS 4
 #endif
+constexpr unsigned kPlainThreads = 512;
 constexpr unsigned kLaneThreads = 1280;  // a server's 8-word lane: three CTAs per SM beside the other lanes' kernels
 template <int NW>
 struct DenseOcc {
@@ -337,7 +340,14 @@ static cudaError_t plan_dense(Ctx &c, Plan &pl, const PlanOpts &o)
         if constexpr (NW == 32) e = plan_variant_fn<192>(c, pl, smem, k_dense<NW, 192>);
         else e = cudaErrorInvalidConfiguration;
         break;
-    case 4: e = plan_variant_fn<128>(c, pl, smem, k_dense<NW, 128>); break;
+    case 4:
+        if constexpr (NW <= 8) {
+            e = o.plain ? plan_variant_fn<128>(c, pl, smem, k_dense<NW, 128, kPlainThreads>)
+                        : plan_variant_fn<128>(c, pl, smem, k_dense<NW, 128>);
+        } else {
+            e = plan_variant_fn<128>(c, pl, smem, k_dense<NW, 128>);
+        }
+        break;
     case 2: e = plan_variant_fn<64>(c, pl, smem, k_dense<NW, 64>); break;
     default: e = plan_variant_fn<32>(c, pl, smem, k_dense<NW, 32>); break;
     }
@@ -523,6 +533,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     PlanOpts po;
     po.wide = job.wide;
     po.half = job.half;
+    po.plain = count == 1;
     po.team = sum_m2 >= 4 * sum_n && sum_n > 0;  // average degree 4 or more: rows walked by teams
     // Lane units (one thread per search unit, vc_lanes.cuh) are opt-in: they
     // execute half the instructions per tree node of warp units but, at 12
@@ -613,6 +624,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     double tl = job.time_limit_s > 0 ? job.time_limit_s : 300.0;
     P.time_limit_ns = (unsigned long long)(tl * 1e9);
     P.pack_after_ns = count == 1 ? pack_after(job.desc[0]) : 0ull;
+    P.dives = count == 1 && job.desc[0].m2 / 16 <= job.desc[0].n;
     P.ring_bias = po.tune ? po.tune->ring_bias : 0;
     P.ring_first = po.tune ? po.tune->ring_first : 0u;
 
