@@ -93,12 +93,12 @@ struct Ctx {
     int coop = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    DevBuf rp, col, inst, st, covers, ctl, seq, data, gws, adj, launches;
-    PinBuf h_st, h_desc, h_covers;
+    DevBuf rp, col, seq, data, gws, adj;
+    DevBuf in, out;      // one launch's descriptors (and a small graph), its control words, states and covers
+    PinBuf h_in, h_out;
     DevBuf ub;     // the upper-bound heuristics (vc_ub.cu)
     DevBuf red;    // reductions of large graphs (struct Reduce)
     PinBuf h_red;
-    unsigned long long h_ctl[vcg::kCtlWords] = {};
     bool stats_on = false;
     bool force_sparse = false;
     Tune tune[kTuneClasses];
@@ -107,6 +107,12 @@ struct Ctx {
     std::vector<unsigned long long> last_stats;
     uint32_t last_num_su = 0;
     Plan last_plan;
+    struct Occ {
+        const void *fn;
+        uint32_t smem;
+        int per_sm;
+    };
+    std::vector<Occ> occ;  // resident CTAs per SM, as asked for once per kernel and shared-memory size
     std::mutex mu;
 };
 
@@ -136,6 +142,8 @@ struct Job {
     const uint32_t *d_rp = nullptr;
     const uint32_t *d_col = nullptr;
     std::vector<vcg::InstDesc> desc;
+    // a host-resident graph that run_job copies with its descriptor (instead of d_rp, d_col)
+    const uint32_t *h_rp = nullptr, *h_col = nullptr;
     double time_limit_s = 0;
     // results
     std::vector<vcg::InstState> st;
@@ -156,6 +164,10 @@ constexpr uint64_t kAdjBytesMax = 4ull << 30;
 
 // The most device memory a context keeps for the upper-bound heuristics (c.ub).
 constexpr uint64_t kUbBytesKept = 1ull << 30;
+
+// Host-resident graphs up to this many bytes go to the device in one copy with
+// their descriptor, from pinned memory; larger ones straight from the caller's.
+constexpr size_t kSmallGraphBytes = 256u << 10;
 
 // The largest graph of the wide dense kernel; it also needs every degree <= 254.
 constexpr uint32_t kWideMaxN = 640;

@@ -49,8 +49,15 @@ constexpr unsigned kMcmThreads = 256;  // 8 search units per CTA
 
 struct McmArgs {
     uint32_t n, nw;
+    uint32_t m2;      // entries, and whether a CTA copies the rows to its shared memory
+    uint32_t rows_in;
     unsigned long long node_limit;
 };
+
+// Rows of up to this many bytes sit in every CTA's shared memory: the walk reads
+// two offsets, a row and an entry per node, one after another, and its first
+// descent is one unit's (planted matching of 1024 vertices 0.45 -> 0.32 ms).
+constexpr uint32_t kMcmRowBytes = 64u << 10;
 
 // Frame depth of one unit: at most n/2 matched entries, plus one.
 __host__ __device__ inline uint32_t mcm_depth(uint32_t n) { return n / 2 + 1; }
@@ -75,11 +82,11 @@ __device__ __forceinline__ bool mcm_next_entry(const uint32_t *rp, const uint32_
     for (;;) {
         const uint32_t nr = mcm_next_row(av, r, lane);
         if (nr == kNone || nr >= n) return false;
-        const uint32_t e0 = nr == cr ? max(ce, __ldg(&rp[nr])) : __ldg(&rp[nr]);
-        const uint32_t e1 = __ldg(&rp[nr + 1]);
+        const uint32_t e0 = nr == cr ? max(ce, rp[nr]) : rp[nr];
+        const uint32_t e1 = rp[nr + 1];
         for (uint32_t eb = e0; eb < e1; eb += 32) {
             const uint32_t ei = eb + lane;
-            const uint32_t u = ei < e1 ? __ldg(&cl[ei]) : 0u;
+            const uint32_t u = ei < e1 ? cl[ei] : 0u;
             const uint32_t word = __shfl_sync(0xffffffffu, av, u >> 5);
             const uint32_t b = __ballot_sync(0xffffffffu, ei < e1 && ((word >> (u & 31u)) & 1u));
             if (b) {
@@ -193,6 +200,14 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
     uint32_t *fp = fe + depth;                       // its row | column << 16
     InstState &st = P.st[0];
     const uint32_t *rp = P.row_ptr, *cl = P.col;
+    if (A.rows_in) {
+        uint32_t *rows = msm + (size_t)(NT / 32) * 2u * depth;
+        for (uint32_t i = threadIdx.x; i <= A.n; i += NT) rows[i] = __ldg(&rp[i]);
+        for (uint32_t i = threadIdx.x; i < A.m2; i += NT) rows[A.n + 1 + i] = __ldg(&cl[i]);
+        rp = rows;
+        cl = rows + A.n + 1;
+        __syncthreads();
+    }
     const unsigned long long deadline = globaltimer() + P.time_limit_ns;
     const uint32_t su = blockIdx.x * (NT / 32) + warp;
     if (su == 0 && lane == 0) atomicCAS(&P.ctl[kT0], 0ull, globaltimer());
@@ -202,7 +217,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
     if (su == 0) {  // the root: every vertex with a neighbour, cursor at entry 0
         for (uint32_t b = 0; b < 32; ++b) {
             const uint32_t v = 32u * lane + b;
-            if (v < A.n && __ldg(&rp[v + 1]) > __ldg(&rp[v])) av |= 1u << b;
+            if (v < A.n && rp[v + 1] > rp[v]) av |= 1u << b;
         }
         have = true;
     }
@@ -270,7 +285,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
                 bot += 1;
                 c_state += 1ull << 32;
             }
-            const uint32_t u = __ldg(&cl[ee]);
+            const uint32_t u = cl[ee];
             if (lane == 0) {
                 fe[level] = ee;
                 fp[level] = er | (u << 16);
@@ -339,7 +354,9 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
     cudaStream_t stream = req->stream ? (cudaStream_t)req->stream : c->stream;
 
     const uint32_t n = g->n, nw = (n + 31) / 32, m2 = 2 * g->m;
-    const uint32_t smem = (kMcmThreads / 32) * 2u * mcm_depth(n) * 4u;
+    const uint64_t row_bytes = 4ull * (n + 1 + (uint64_t)m2);
+    const bool rows_in = row_bytes <= kMcmRowBytes;
+    const uint32_t smem = (kMcmThreads / 32) * 2u * mcm_depth(n) * 4u + (rows_in ? (uint32_t)row_bytes : 0u);
     auto fn = k_mcm<kMcmThreads>;
     int per_sm = 0;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -351,18 +368,29 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
     uint32_t q = 1024;
     while (q < 2 * num_su) q <<= 1;
     const uint32_t stride = (4 + nw + 3) / 4 * 4;
-    if (c->rp.ensure(4ull * (n + 1)) || c->col.ensure(4ull * std::max<uint32_t>(m2, 1)) ||
-        c->st.ensure(sizeof(InstState)) || c->ctl.ensure(sizeof(unsigned long long) * kCtlWords) ||
-        c->seq.ensure(sizeof(unsigned long long) * q) || c->data.ensure(4ull * q * stride))
+    // one piece of device memory, mirrored in pinned: control words, state, rows;
+    // the first two come back
+    const size_t st_at = sizeof(unsigned long long) * kCtlWords, rp_at = st_at + sizeof(InstState),
+                 bytes = rp_at + 4ull * (n + 1 + (uint64_t)m2);
+    const bool small = bytes <= kSmallGraphBytes;
+    if (c->out.ensure(bytes) || c->h_out.ensure(small ? bytes : rp_at) || c->seq.ensure(sizeof(unsigned long long) * q) ||
+        c->data.ensure(4ull * q * stride))
         return VC_ERR_NOMEM;
+    uint8_t *d = (uint8_t *)c->out.p, *h = (uint8_t *)c->h_out.p;
     InstState s0;
     memset(&s0, 0, sizeof(s0));
     s0.act = 1;  // the root
     s0.cover_size = kNone;
-    bool ok = cudaMemcpyAsync(c->rp.p, g->row_ptr, 4ull * (n + 1), cudaMemcpyHostToDevice, stream) == cudaSuccess &&
-              (m2 == 0 || cudaMemcpyAsync(c->col.p, g->col, 4ull * m2, cudaMemcpyHostToDevice, stream) == cudaSuccess) &&
-              cudaMemcpyAsync(c->st.p, &s0, sizeof(s0), cudaMemcpyHostToDevice, stream) == cudaSuccess &&
-              cudaMemsetAsync(c->ctl.p, 0, sizeof(unsigned long long) * kCtlWords, stream) == cudaSuccess;
+    memset(h, 0, st_at);
+    memcpy(h + st_at, &s0, sizeof(s0));
+    if (small) {
+        memcpy(h + rp_at, g->row_ptr, 4ull * (n + 1));
+        if (m2) memcpy(h + rp_at + 4ull * (n + 1), g->col, 4ull * m2);
+    }
+    bool ok = cudaMemcpyAsync(d, h, small ? bytes : rp_at, cudaMemcpyHostToDevice, stream) == cudaSuccess;
+    if (!small)
+        ok = ok && cudaMemcpyAsync(d + rp_at, g->row_ptr, 4ull * (n + 1), cudaMemcpyHostToDevice, stream) == cudaSuccess &&
+             (m2 == 0 || cudaMemcpyAsync(d + rp_at + 4ull * (n + 1), g->col, 4ull * m2, cudaMemcpyHostToDevice, stream) == cudaSuccess);
     if (!ok) {
         cudaStreamSynchronize(stream);
         return VC_ERR_CUDA;
@@ -378,12 +406,12 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
     }
     Params P;
     memset(&P, 0, sizeof(P));
-    P.row_ptr = (const uint32_t *)c->rp.p;
-    P.col = (const uint32_t *)c->col.p;
-    P.st = (InstState *)c->st.p;
+    P.row_ptr = (const uint32_t *)(d + rp_at);
+    P.col = P.row_ptr + n + 1;
+    P.st = (InstState *)(d + st_at);
     P.count = 1;
     P.num_su = num_su;
-    P.ctl = (unsigned long long *)c->ctl.p;
+    P.ctl = (unsigned long long *)d;
     P.pool_seq = (unsigned long long *)c->seq.p;
     P.pool_data = (uint32_t *)c->data.p;
     P.q_mask = q - 1;
@@ -393,6 +421,8 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
     McmArgs A;
     A.n = n;
     A.nw = nw;
+    A.m2 = m2;
+    A.rows_in = rows_in ? 1u : 0u;
     A.node_limit = req->node_limit;
     Plan pl;
     pl.fn = (const void *)fn;
@@ -409,12 +439,11 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
         cudaLaunchKernel((const void *)fn, dim3(grid), dim3(kMcmThreads), args, smem, stream) == cudaSuccess;
     cudaEventRecord(c->ev1, stream);
     g_launches += 2;
-    InstState s1;
-    unsigned long long abort_word = 0;
-    ok = launched && cudaMemcpyAsync(&s1, c->st.p, sizeof(s1), cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
-         cudaMemcpyAsync(&abort_word, (unsigned long long *)c->ctl.p + kAbort, sizeof(abort_word),
-                         cudaMemcpyDeviceToHost, stream) == cudaSuccess;
+    ok = launched && cudaMemcpyAsync(h, d, rp_at, cudaMemcpyDeviceToHost, stream) == cudaSuccess;
     if (cudaStreamSynchronize(stream) != cudaSuccess || !ok) return VC_ERR_CUDA;
+    InstState s1;
+    memcpy(&s1, h + st_at, sizeof(s1));
+    const unsigned long long abort_word = ((const unsigned long long *)h)[kAbort];
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     out->size = s1.best;

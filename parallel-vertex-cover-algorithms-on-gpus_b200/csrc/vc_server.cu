@@ -69,9 +69,9 @@ struct Done {
 
 constexpr uint32_t kSubQ = 1u << 16;  // submission queue entries (power of two)
 constexpr uint32_t kAdmit = 256;      // requests per admission
-// Pinned bytes of an admission's graphs.  Fixed at creation: freeing pinned memory
+// Pinned bytes of an admission's graphs.  Made with the lane: freeing pinned memory
 // waits for the device, which a running lane keeps busy.
-constexpr size_t kStageBytes = 2u << 20;
+constexpr size_t kStageBytes = 512u << 10;
 
 }  // namespace
 
@@ -83,8 +83,11 @@ struct SrvLane {
     uint64_t arena_cap = 0;
     Plan pl;
     uint32_t q = 0;
-    DevBuf desc, st, covers, ctl, seq, data, gws, subq, arena;
-    PinBuf stage;  // what an admission copies
+    DevBuf slab;  // all of the lane's device memory; the pieces below point into it
+    struct Piece {
+        void *p = nullptr;
+    } desc, st, covers, ctl, seq, data, gws, subq, arena;
+    uint8_t *stage = nullptr;  // what an admission copies (pinned, behind h_res)
     uint32_t *h_res = nullptr, *d_res = nullptr;
     uint32_t res_words = 0;
     // host state (guarded by mu)
@@ -290,7 +293,7 @@ uint32_t admit(SrvLane *s, std::unique_lock<std::mutex> &lk, bool &arena_full)
     lk.unlock();
     bool ok = true;
     {
-        uint8_t *h = (uint8_t *)s->stage.p;
+        uint8_t *h = s->stage;
         uint32_t *w = (uint32_t *)h;
         const size_t at_desc = kStageBytes, at_slot = at_desc + sizeof(InstDesc) * kAdmit, at_tail = at_slot + 4 * kAdmit;
         memcpy(h + at_desc, descs.data(), sizeof(InstDesc) * batch.size());
@@ -486,16 +489,7 @@ void lane_destroy(SrvLane *s)
     if (!s) return;
     lane_stop(s);
     if (s->loop.joinable()) s->loop.join();
-    s->desc.release();
-    s->st.release();
-    s->covers.release();
-    s->ctl.release();
-    s->seq.release();
-    s->data.release();
-    s->gws.release();
-    s->subq.release();
-    s->arena.release();
-    s->stage.release();
+    s->slab.release();
     if (s->h_res) cudaFreeHost(s->h_res);
     if (s->kstream) cudaStreamDestroy(s->kstream);
     if (s->cstream) cudaStreamDestroy(s->cstream);
@@ -523,16 +517,32 @@ vc_status lane_create(Ctx *c, uint64_t budget, uint32_t slots, uint32_t max_n, c
     s->arena_free.emplace(0, budget);
     bool ok = cudaStreamCreateWithFlags(&s->kstream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaStreamCreateWithFlags(&s->cstream, cudaStreamNonBlocking) == cudaSuccess;
-    ok = ok && !s->desc.ensure(sizeof(InstDesc) * s->slots) && !s->st.ensure(sizeof(InstState) * s->slots) &&
-         !s->covers.ensure(4ull * s->slots * s->nw_max) && !s->ctl.ensure(sizeof(unsigned long long) * kCtlWords) &&
-         !s->seq.ensure(sizeof(unsigned long long) * s->q) && !s->data.ensure(4ull * s->q * s->pl.stride) &&
-         !s->subq.ensure(4ull * kSubQ) && !s->arena.ensure(budget) &&
-         (!s->pl.global_ws || !s->gws.ensure((size_t)s->pl.num_su * s->pl.su_bytes));
+    // One allocation of device and one of pinned memory: each of the nine pieces by
+    // itself costs its call and, at the end, a wait for the device.
+    size_t bytes = 0;
+    std::vector<std::pair<SrvLane::Piece *, size_t>> pieces;
+    auto piece = [&](SrvLane::Piece &p, size_t b) {
+        pieces.emplace_back(&p, bytes);
+        bytes += (b + 255) / 256 * 256;
+    };
+    piece(s->desc, sizeof(InstDesc) * s->slots);
+    piece(s->st, sizeof(InstState) * s->slots);
+    piece(s->covers, 4ull * s->slots * s->nw_max);
+    piece(s->ctl, sizeof(unsigned long long) * kCtlWords);
+    piece(s->seq, sizeof(unsigned long long) * s->q);
+    piece(s->data, 4ull * s->q * s->pl.stride);
+    piece(s->subq, 4ull * kSubQ);
+    if (s->pl.global_ws) piece(s->gws, (size_t)s->pl.num_su * s->pl.su_bytes);
+    piece(s->arena, budget);
+    ok = ok && !s->slab.ensure(bytes);
+    if (ok)
+        for (auto &p : pieces) p.first->p = (uint8_t *)s->slab.p + p.second;
     ok = ok && cudaMemset(s->ctl.p, 0, sizeof(unsigned long long) * kCtlWords) == cudaSuccess;
-    ok = ok && !s->stage.ensure(kStageBytes + (sizeof(InstDesc) + 4) * kAdmit + sizeof(unsigned long long));
-    const size_t res_bytes = 4ull * s->slots * s->res_words;
-    ok = ok && cudaHostAlloc((void **)&s->h_res, res_bytes, cudaHostAllocMapped) == cudaSuccess;
+    const size_t res_bytes = (4ull * s->slots * s->res_words + 255) / 256 * 256;
+    const size_t stage_bytes = kStageBytes + (sizeof(InstDesc) + 4) * kAdmit + sizeof(unsigned long long);
+    ok = ok && cudaHostAlloc((void **)&s->h_res, res_bytes + stage_bytes, cudaHostAllocMapped) == cudaSuccess;
     ok = ok && cudaHostGetDevicePointer((void **)&s->d_res, s->h_res, 0) == cudaSuccess;
+    s->stage = (uint8_t *)s->h_res + res_bytes;
     if (!ok) {
         lane_destroy(s);
         return VC_ERR_NOMEM;

@@ -258,21 +258,25 @@ Ctx *get_ctx(int dev, vc_status *err)
 }
 
 // ---------------------------------------------------------------- sizing
-// Resident CTAs per SM of `fn` with `smem` bytes of dynamic shared memory (0 on error).
+// Resident CTAs per SM of `fn` with `smem` bytes of dynamic shared memory (0 on
+// error).  The answer is a property of the kernel and the device: it is kept; the
+// attribute is set every time, since a launch elsewhere may have lowered it.
 template <unsigned NT, class F>
-static int ctas_per_sm(F fn, uint32_t smem)
+static int ctas_per_sm(Ctx &c, F fn, uint32_t smem)
 {
     int per_sm = 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)NT, smem) != cudaSuccess)
-        return 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    for (const Ctx::Occ &o : c.occ)
+        if (o.fn == (const void *)fn && o.smem == smem) return o.per_sm;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)NT, smem) != cudaSuccess) return 0;
+    if (c.occ.size() < 256) c.occ.push_back({(const void *)fn, smem, per_sm});
     return per_sm;
 }
 
 template <unsigned NT, class F>
 static cudaError_t plan_variant_fn(Ctx &c, Plan &pl, uint32_t smem_per_block, F fn)
 {
-    const int per_sm = ctas_per_sm<NT>(fn, smem_per_block);
+    const int per_sm = ctas_per_sm<NT>(c, fn, smem_per_block);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     pl.fn = (const void *)fn;
     pl.block = NT;
@@ -289,8 +293,8 @@ static cudaError_t plan_variant(Ctx &c, Plan &pl, uint32_t smem_per_block)
 {
     if constexpr (G::kTeam) {
         auto roomy = k_search<G, NT, kRoomyThreadsPerSM>;
-        const int r = ctas_per_sm<NT>(roomy, smem_per_block);
-        if (r > 0 && r >= ctas_per_sm<NT>(k_search<G, NT>, smem_per_block))
+        const int r = ctas_per_sm<NT>(c, roomy, smem_per_block);
+        if (r > 0 && r >= ctas_per_sm<NT>(c, k_search<G, NT>, smem_per_block))
             return plan_variant_fn<NT>(c, pl, smem_per_block, roomy);
     }
     return plan_variant_fn<NT>(c, pl, smem_per_block, k_search<G, NT>);
@@ -551,15 +555,22 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     while (q > 64 && (size_t)q * stride * 4 > ring_cap_bytes) q >>= 1;
 
     size_t gws_bytes = pl.global_ws ? (size_t)pl.num_su * pl.su_bytes : 0;
-    if (c.inst.ensure(sizeof(InstDesc) * count) || c.st.ensure(sizeof(InstState) * count) ||
-        c.covers.ensure(sizeof(uint32_t) * std::max<uint32_t>(cover_words, 1)) ||
-        c.ctl.ensure(sizeof(unsigned long long) * kCtlWords) || c.seq.ensure(sizeof(unsigned long long) * q) ||
-        c.data.ensure((size_t)q * stride * 4) || c.launches.ensure(sizeof(unsigned long long)) ||
-        (gws_bytes && c.gws.ensure(gws_bytes)))
+    // One piece in (the descriptors, with a small host-resident graph) and one out
+    // (control words, states, covers), each mirrored in pinned memory: one copy each.
+    const size_t rp_at = sizeof(InstDesc) * (size_t)count;
+    const size_t col_at = rp_at + (job.h_rp ? 4ull * (job.desc[0].n + 1) : 0);
+    const size_t in_bytes = col_at + (job.h_rp ? 4ull * job.desc[0].m2 : 0);
+    const size_t st_at = sizeof(unsigned long long) * kCtlWords, covers_at = st_at + sizeof(InstState) * (size_t)count;
+    const size_t out_bytes = covers_at + sizeof(uint32_t) * (size_t)cover_words;
+    if (c.in.ensure(in_bytes) || c.out.ensure(out_bytes) || c.seq.ensure(sizeof(unsigned long long) * q) ||
+        c.data.ensure((size_t)q * stride * 4) || (gws_bytes && c.gws.ensure(gws_bytes)))
         return VC_ERR_NOMEM;
-    if (c.h_st.ensure(sizeof(InstState) * count) || c.h_desc.ensure(sizeof(InstDesc) * count) ||
-        c.h_covers.ensure(sizeof(uint32_t) * std::max<uint32_t>(cover_words, 1)))
-        return VC_ERR_NOMEM;
+    if (c.h_in.ensure(in_bytes) || c.h_out.ensure(out_bytes)) return VC_ERR_NOMEM;
+    uint8_t *d_in = (uint8_t *)c.in.p, *d_out = (uint8_t *)c.out.p;
+    if (job.h_rp) {
+        job.d_rp = (const uint32_t *)(d_in + rp_at);
+        job.d_col = (const uint32_t *)(d_in + col_at);
+    }
 
     // bitmap rows for the dense kernels, up to a bound on what they take (above it
     // the search units make them from the CSR when they stage a graph)
@@ -572,16 +583,23 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
         }
         if (4 * adj_words > kAdjBytesMax || c.adj.ensure(4 * adj_words)) adj_words = 0;
     }
-    memcpy(c.h_desc.p, job.desc.data(), sizeof(InstDesc) * count);
-    cudaMemcpyAsync(c.inst.p, c.h_desc.p, sizeof(InstDesc) * count, cudaMemcpyHostToDevice, stream);
+    {
+        uint8_t *h = (uint8_t *)c.h_in.p;
+        memcpy(h, job.desc.data(), sizeof(InstDesc) * count);
+        if (job.h_rp) {
+            memcpy(h + rp_at, job.h_rp, col_at - rp_at);
+            if (in_bytes > col_at) memcpy(h + col_at, job.h_col, in_bytes - col_at);
+        }
+        cudaMemcpyAsync(d_in, h, in_bytes, cudaMemcpyHostToDevice, stream);
+    }
     PrepareArgs A;
-    A.ctl = (unsigned long long *)c.ctl.p;
+    A.ctl = (unsigned long long *)d_out;
     A.seq = (unsigned long long *)c.seq.p;
     A.q = q;
-    A.covers = (uint32_t *)c.covers.p;
+    A.covers = (uint32_t *)(d_out + covers_at);
     A.cover_words = cover_words;
-    A.st = (InstState *)c.st.p;
-    A.inst = (const InstDesc *)c.inst.p;
+    A.st = (InstState *)(d_out + st_at);
+    A.inst = (const InstDesc *)d_in;
     A.count = count;
     A.row_ptr = job.d_rp;
     A.col = job.d_col;
@@ -600,13 +618,13 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     memset(&P, 0, sizeof(P));
     P.row_ptr = job.d_rp;
     P.col = job.d_col;
-    P.inst = (const InstDesc *)c.inst.p;
-    P.st = (InstState *)c.st.p;
-    P.covers = (uint32_t *)c.covers.p;
+    P.inst = A.inst;
+    P.st = A.st;
+    P.covers = A.covers;
     P.adj = A.adj;
     P.count = count;
     P.num_su = pl.num_su;
-    P.ctl = (unsigned long long *)c.ctl.p;
+    P.ctl = A.ctl;
     P.pool_seq = (unsigned long long *)c.seq.p;
     P.pool_data = (uint32_t *)c.data.p;
     P.q_mask = q - 1;
@@ -634,18 +652,15 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     if (e != cudaSuccess) return VC_ERR_CUDA;
     g_launches += 1;
     cudaEventRecord(c.ev1, stream);
-    cudaMemcpyAsync(c.h_st.p, c.st.p, sizeof(InstState) * count, cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(c.h_covers.p, c.covers.p, sizeof(uint32_t) * std::max<uint32_t>(cover_words, 1),
-                    cudaMemcpyDeviceToHost, stream);
-    unsigned long long abort_flag = 0;
-    cudaMemcpyAsync(c.h_ctl, c.ctl.p, sizeof(unsigned long long) * kCtlWords, cudaMemcpyDeviceToHost, stream);
+    cudaMemcpyAsync(c.h_out.p, d_out, out_bytes, cudaMemcpyDeviceToHost, stream);
     if (cudaStreamSynchronize(stream) != cudaSuccess) return VC_ERR_CUDA;
-    abort_flag = c.h_ctl[kAbort];
-    job.t0 = c.h_ctl[kT0];
+    const uint8_t *h_out = (const uint8_t *)c.h_out.p;
+    const unsigned long long *h_ctl = (const unsigned long long *)h_out;
+    job.t0 = h_ctl[kT0];
     cudaEventElapsedTime(&job.kernel_ms, c.ev0, c.ev1);
-    job.aborted = abort_flag != 0;
-    job.st.assign((InstState *)c.h_st.p, (InstState *)c.h_st.p + count);
-    job.covers.assign((uint32_t *)c.h_covers.p, (uint32_t *)c.h_covers.p + std::max<uint32_t>(cover_words, 1));
+    job.aborted = h_ctl[kAbort] != 0;
+    job.st.assign((const InstState *)(h_out + st_at), (const InstState *)(h_out + st_at) + count);
+    job.covers.assign((const uint32_t *)(h_out + covers_at), (const uint32_t *)(h_out + covers_at) + cover_words);
     job.plan = pl;
     if (c.stats_on) {
         c.last_stats.resize((size_t)kStatWords * pl.num_su);
@@ -921,15 +936,20 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
     std::lock_guard<std::mutex> lk(c->mu);
     cudaStream_t stream = req->stream ? (cudaStream_t)req->stream : c->stream;
 
+    // a large graph: its root is reduced by the whole chip, the search gets the rest
+    const bool large = g->n > kHalfMaxN && !c->force_sparse && 2ull * g->m < kNone;
+    const size_t rp_b = sizeof(uint32_t) * ((size_t)g->n + 1), col_b = sizeof(uint32_t) * 2 * (size_t)g->m;
     Job job;
     if (dev_in) {
         job.d_rp = g->row_ptr;
         job.d_col = g->col;
+    } else if (!large && rp_b + col_b <= kSmallGraphBytes) {
+        job.h_rp = g->row_ptr;
+        job.h_col = g->col;
     } else {
-        size_t rp_b = sizeof(uint32_t) * ((size_t)g->n + 1), col_b = sizeof(uint32_t) * std::max<size_t>(2 * (size_t)g->m, 1);
-        if (c->rp.ensure(rp_b) || c->col.ensure(col_b)) return VC_ERR_NOMEM;
+        if (c->rp.ensure(rp_b) || c->col.ensure(std::max<size_t>(col_b, 4))) return VC_ERR_NOMEM;
         cudaMemcpyAsync(c->rp.p, g->row_ptr, rp_b, cudaMemcpyHostToDevice, stream);
-        if (g->m) cudaMemcpyAsync(c->col.p, g->col, sizeof(uint32_t) * 2 * (size_t)g->m, cudaMemcpyHostToDevice, stream);
+        if (g->m) cudaMemcpyAsync(c->col.p, g->col, col_b, cudaMemcpyHostToDevice, stream);
         job.d_rp = (const uint32_t *)c->rp.p;
         job.d_col = (const uint32_t *)c->col.p;
     }
@@ -938,8 +958,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
     InstDesc d{};
     float reduce_ms = 0;
     std::vector<Reduce> red;
-    if (g->n > kHalfMaxN && !c->force_sparse && 2ull * g->m < kNone) {
-        // a large graph: its root is reduced by the whole chip, the search gets the rest
+    if (large) {
         Reduce r;
         r.rp = job.d_rp;
         r.cl = job.d_col;
