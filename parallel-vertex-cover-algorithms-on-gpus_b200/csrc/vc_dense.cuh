@@ -918,6 +918,48 @@ __device__ __forceinline__ void load_root(DSU<NW> &s)
     s.pending = kPendRecount;  // the node's settling counts the degrees
 }
 
+// Root `v` of a split graph: the vertices of larger degree (then of lower index) are
+// in the cover and v is not, so its neighbours are too.  The n roots part the covers
+// by their first vertex in that order that stays out.  From the single root of a
+// dense graph the search goes down a spine of nearly n nodes, "take v" each, before
+// its first leaf, one after another (300 vertices of density 0.75: 279 nodes and
+// most of the solve's 1.7 ms); the children that it would leave behind are these
+// roots, and all CTAs take them up at once.
+template <int NW>
+__device__ __forceinline__ void load_split_root(DSU<NW> &s, uint32_t v)
+{
+    const unsigned lane = lane_id();
+    auto degree = [&](uint32_t u) {
+        uint32_t r[NW], d = 0;
+        load_row_at<NW>(s.adj, u, r);
+#pragma unroll
+        for (int i = 0; i < NW; ++i) d += __popc(r[i]);
+        return d;
+    };
+    const uint32_t dv = degree(v);
+    uint32_t keep = 0;
+    for (uint32_t w = 0; w < s.nw; ++w) {
+        const uint32_t u = 32u * w + lane;
+        bool in = false;
+        if (u < s.n) {
+            const uint32_t du = degree(u);
+            in = du < dv || (du == dv && u >= v);
+        }
+        const uint32_t x = __ballot_sync(0xffffffffu, in);
+        if (lane == w) keep = x;
+    }
+    if (lane < (uint32_t)NW) {
+        keep &= ~s.adj[Rows<NW>::at(v, lane)];
+        s.lsm()[lane] = keep;
+        s.marks()[lane] = 0;
+    }
+    const uint32_t live = __reduce_add_sync(0xffffffffu, __popc(keep));
+    s.top = 0;
+    s.base_del = s.n - live;
+    __syncwarp();
+    s.pending = kPendRecount;
+}
+
 // From a received live bitmap in s.bits().
 template <class G, int NW>
 __device__ __forceinline__ void rebuild(DSU<NW> &s)
@@ -1313,13 +1355,15 @@ __device__ bool acquire_cta(DSU<NW> &s, const Params &P, CtaPool &cp, uint32_t *
         if (res == 3) return false;
         if (res == 4) {  // a new graph root for the whole CTA
             slot = G::bcast(slot);
-            const uint32_t key = __ldcg(&P.inst[slot].key);
+            const uint32_t inst = P.split ? 0u : slot;
+            const uint32_t key = __ldcg(&P.inst[inst].key);
             if (vld(&cp.hdr[kCpStaged]) != key) {
-                stage_graph<NW>(adj, P, slot);
+                stage_graph<NW>(adj, P, inst);
                 if (lane == 0) cp.hdr[kCpStaged] = key;
             }
-            bind_graph<G>(s, P, slot);
-            load_root<G>(s);
+            bind_graph<G>(s, P, inst);
+            if (P.split) load_split_root<NW>(s, slot);
+            else load_root<G>(s);
             s.stat.roots += 1;
             return true;
         }

@@ -838,7 +838,7 @@ __device__ __forceinline__ bool claim_root(const Params &P, uint32_t &slot)
 {
     if (!P.server) {
         const uint32_t i = (uint32_t)atomicAdd(&P.ctl[kCursor], 1ull);
-        if (i < P.count) { slot = i; return true; }
+        if (i < (P.split ? P.split : P.count)) { slot = i; return true; }
         return false;
     }
     for (int it = 0; it < 4; ++it) {

@@ -89,6 +89,7 @@ struct Params {
     unsigned long long *stats;    // per-SU counters (kStatWords each), null = off
     unsigned long long time_limit_ns;
     unsigned long long pack_after_ns;  // dense kernels: use the packing bound once the launch has run this long
+    uint32_t split;     // dense kernels, one graph: it is searched from this many roots (its n), 0 = from one
     uint32_t dives;     // dense kernels: first blocks start with greedy dives
     int32_t ring_bias;  // give work to the global ring while idle CTAs minus queued records exceed this (< 0: keep a surplus queued)
     uint32_t ring_first;  // when both idle sibling warps and idle CTAs wait: 0 local pool first, 1 ring first, 2 alternate
