@@ -34,12 +34,15 @@
 // search stops with "not found".
 //
 // What bounds it is one deletion's chain, whatever the size: find the vertex, read
-// its row, the last entries of its neighbours' rows, move them, and four block
-// barriers.  So the bitmaps, degrees and offsets sit in shared memory where they
-// fit (graphs of up to some 26,000 vertices; the bitmaps alone above).  RemoveMax
-// and RemoveEdge on a power-law graph of 12,000 vertices: 18.5 -> 6.5 and 21.6 -> 6.5 ms;
-// of 100,000: 208 -> 75 and 236 -> 76 ms (before: 1024 threads, rows read and their
-// neighbours of neighbours marked at every deletion, state in global memory).
+// its row, the last entries of its neighbours' rows, move them -- three dependent
+// reads from L2.  The rest is kept off it: bitmaps, degrees, offsets and the records
+// of the last deletions sit in shared memory where they fit (graphs of up to some
+// 14,000 vertices; the bitmaps alone above), and the leaf rule, most deletions of a
+// sparse graph, is one warp's without a barrier of the block.  RemoveMax and
+// RemoveEdge on a power-law graph of 12,000 vertices: 18.5 -> 5.3 and 21.6 -> 5.4 ms;
+// of 100,000: 208 -> 72 and 236 -> 72 ms (before: 1024 threads, rows read and their
+// neighbours of neighbours marked at every deletion, state in global memory; with
+// the block's barriers in the leaf rule 6.3 ms on the smaller).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -83,6 +86,7 @@ struct UbParams {
 };
 
 constexpr uint32_t kMaxBlock = 1024;  // vertices per cached maximum
+constexpr int kWarpDelete = 96;       // neighbours up to which one warp deletes a leaf's neighbour
 
 // deg1, two, dirty, moved and deg1's summary, in words; then the cached maxima (two
 // words each), then degrees and offsets where they fit too.
@@ -92,10 +96,11 @@ __host__ __device__ inline uint64_t ub_bitmap_words(uint32_t n)
     return (4 * nw + (nw + 31) / 32 + 1) / 2 * 2;
 }
 __host__ __device__ inline uint64_t ub_set_words(uint32_t n) { return ub_bitmap_words(n) + 2ull * ((n + kMaxBlock - 1) / kMaxBlock); }
-__host__ __device__ inline uint64_t ub_all_words(uint32_t n) { return ub_set_words(n) + 2ull * n + 1; }
+__host__ __device__ inline uint64_t ub_all_words(uint32_t n) { return ub_set_words(n) + 4ull * n + 1; }
 
 struct UbShared {
     uint32_t x;          // the vertex to delete, or kInf
+    uint32_t minimum, stamp;  // the block's, while one warp deletes
     uint32_t found;      // block search result
     uint32_t cnt1;       // vertices of degree 1
     uint32_t any;        // dirty or moved not empty
@@ -133,14 +138,22 @@ __device__ __forceinline__ void ub_set1(const Ub &g, UbShared &sh, uint32_t v)
 // row; if z loses x too and that mate is what z moves, it is found where z's x was
 // (both ends of such a pair then write the same).  `stamp` numbers these steps of a
 // graph from 1.  The block has passed a barrier since x was chosen, and passes one
-// after this before it reads what this changed.
-__device__ void ub_delete(const Ub &g, UbShared &sh, uint32_t x, uint32_t &stamp)
+// after this before it reads what this changed.  With Warp it is one warp's work,
+// and its barriers are the warp's.
+template <bool Warp>
+__device__ __forceinline__ void ub_delete(const Ub &g, UbShared &sh, uint32_t x, uint32_t &stamp)
 {
+    constexpr int kStep = Warp ? 32 : (int)kUbThreads;
+    const int me = Warp ? (int)lane_of() : (int)threadIdx.x;
+    auto barrier = [] {
+        if constexpr (Warp) __syncwarp();
+        else __syncthreads();
+    };
     const int dx = g.deg[x];
     const uint32_t bx = g.rp[x];
-    for (int base = 0; base < dx; base += (int)kUbThreads) {
+    for (int base = 0; base < dx; base += kStep) {
         ++stamp;
-        const int t = base + (int)threadIdx.x;
+        const int t = base + me;
         const bool mine = t < dx;
         uint32_t w = 0, pos = 0, z = x, zm = 0;
         int dw = 0;
@@ -153,7 +166,7 @@ __device__ void ub_delete(const Ub &g, UbShared &sh, uint32_t x, uint32_t &stamp
             zm = g.mate[last];
             g.gone[w] = make_uint2(stamp, pos);
         }
-        __syncthreads();
+        barrier();
         if (mine && z != x) {
             const uint2 gz = g.gone[z];
             if (gz.x == stamp && zm == g.rp[z] + (uint32_t)g.deg[z] - 1u) zm = gz.y;
@@ -161,7 +174,7 @@ __device__ void ub_delete(const Ub &g, UbShared &sh, uint32_t x, uint32_t &stamp
             g.mate[pos] = zm;
             g.mate[zm] = pos;
         }
-        __syncthreads();
+        barrier();
         if (mine) {
             g.deg[w] = dw - 1;
             if (dw == 3) {
@@ -176,9 +189,9 @@ __device__ void ub_delete(const Ub &g, UbShared &sh, uint32_t x, uint32_t &stamp
             }
             ub_put(g.mv, w);
         }
-        if (base + (int)kUbThreads < dx) __syncthreads();
+        if (base + kStep < dx) barrier();
     }
-    if (threadIdx.x == 0) {
+    if (me == 0) {
         if (dx == 1) {
             ub_drop(g.d1, x);
             atomicSub(&sh.cnt1, 1u);
@@ -292,7 +305,8 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
     g.mv = sets + 3 * g.nw;
     g.s1 = sets + 4 * g.nw;
     g.bmax = reinterpret_cast<unsigned long long *>(sets + ub_bitmap_words(n));
-    uint32_t *rp_in = ub_smem + ub_set_words(n);
+    uint32_t *rp_in = ub_smem + ub_set_words(n) + 2ull * n;
+    if (all_in) g.gone = reinterpret_cast<uint2 *>(ub_smem + ub_set_words(n));
     g.deg = all_in ? reinterpret_cast<int32_t *>(rp_in + n + 1) : deg0;
     g.rp = all_in ? rp_in : rp0;
     const uint32_t m2 = n ? rp0[n] : 0u;
@@ -333,29 +347,46 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
     for (;;) {
         if (P.mode == 1 && !(vertex < n && remaining > 0)) break;
         const uint32_t before = minimum;
-        // leaf rule to its fixpoint: passes in index order while a pass acts
+        // leaf rule to its fixpoint: passes in index order while a pass acts.  One
+        // warp runs it, with no barrier of the block, until a vertex of many
+        // neighbours is due.
         {
             uint32_t p = 0;  // (in warp 0; so is `changed`)
             bool changed = false;
             for (;;) {
                 __syncthreads();  // the deletion before this is complete
-                if (sh.cnt1 == 0) break;  // no pass can act any more
                 if (warp_of() == 0) {
-                    uint32_t i = ub_next_leaf(g, p);
-                    if (i == kInf && changed) {
-                        changed = false;
-                        i = ub_next_leaf(g, 0);
-                    }
-                    if (i != kInf) {
+                    uint32_t x = kInf;
+                    while (*(volatile uint32_t *)&sh.cnt1 != 0) {  // else no pass can act any more
+                        uint32_t i = ub_next_leaf(g, p);
+                        if (i == kInf && changed) {
+                            changed = false;
+                            i = ub_next_leaf(g, 0);
+                        }
+                        if (i == kInf) break;
                         changed = true;
                         p = i + 1;
+                        const uint32_t only = *(volatile uint32_t *)&g.dst[g.rp[i]];  // its only live neighbour
+                        if (g.deg[only] > kWarpDelete) {
+                            x = only;
+                            break;
+                        }
+                        ub_delete<true>(g, sh, only, stamp);
+                        minimum += 1;
+                        __syncwarp();
                     }
-                    if (lane_of() == 0) sh.x = i == kInf ? kInf : g.dst[g.rp[i]];  // its only live neighbour
+                    if (lane_of() == 0) {
+                        sh.x = x;
+                        sh.minimum = minimum;
+                        sh.stamp = stamp;
+                    }
                 }
                 __syncthreads();
                 const uint32_t x = sh.x;
+                minimum = sh.minimum;
+                stamp = sh.stamp;
                 if (x == kInf) break;
-                ub_delete(g, sh, x, stamp);
+                ub_delete<false>(g, sh, x, stamp);
                 minimum += 1;
             }
         }
@@ -399,9 +430,9 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
             uint32_t a = 0, b = 0;
             ub_fires(g.rp, g.dst, g.deg, fire, &a, &b);
             __syncthreads();  // every thread has both
-            ub_delete(g, sh, a, stamp);
+            ub_delete<false>(g, sh, a, stamp);
             __syncthreads();
-            ub_delete(g, sh, b, stamp);
+            ub_delete<false>(g, sh, b, stamp);
             minimum += 2;
         }
         if (P.mode == 0) {
@@ -434,7 +465,7 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
             }
             const unsigned long long k = sh.amax;
             if (k == 0) break;
-            ub_delete(g, sh, ~(uint32_t)k, stamp);
+            ub_delete<false>(g, sh, ~(uint32_t)k, stamp);
             minimum += 1;
         } else {
             // on to the next live vertex at once if the rules had nothing to do: they
@@ -453,9 +484,9 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
                 remaining -= (uint32_t)g.deg[u];
                 ++remaining;
                 __syncthreads();  // every thread has them
-                ub_delete(g, sh, vertex, stamp);
+                ub_delete<false>(g, sh, vertex, stamp);
                 __syncthreads();
-                ub_delete(g, sh, u, stamp);
+                ub_delete<false>(g, sh, u, stamp);
                 minimum += 2;
             }
             ++vertex;

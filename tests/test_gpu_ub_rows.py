@@ -42,7 +42,7 @@ def test_rows_longer_than_a_block_and_crossing_rows(n, hubs):
         assert ubs[0] == want and np.array_equal(covers[0], np.asarray(mask, dtype=bool))
 
 
-@pytest.mark.parametrize("n", [26000, 30000])
+@pytest.mark.parametrize("n", [14000, 14100, 26000, 30000])
 def test_around_what_shared_memory_holds(n):
     """The largest graphs whose degrees and offsets sit in shared memory, and those that keep their bitmaps only."""
     g = W.gnp(n, 2.6 / (n - 1), n)
