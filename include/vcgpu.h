@@ -39,9 +39,9 @@ typedef enum vc_instance {
     VC_PVC = 1  /* parameterized vertex cover, decision size <= k (`-i pvc -k K`) */
 } vc_instance;
 
-/* vc_request.flags.  Host-resident graphs are checked on the host (monotone
- * offsets, ids < n, no self loop or duplicate, sorted symmetric rows) unless
- * VC_FLAG_NO_VALIDATE.  Device-resident graphs (VC_FLAG_DEVICE_INPUT, and
+/* vc_request.flags.  Host-resident graphs are checked (monotone offsets, ids < n,
+ * no self loop or duplicate, sorted symmetric rows; on the host, or by a kernel
+ * above 2048 entries) unless VC_FLAG_NO_VALIDATE.  Device-resident graphs (VC_FLAG_DEVICE_INPUT, and
  * vc_solve_batch_device) cannot be read by the host: a kernel checks the layout
  * the search relies on for memory safety -- row_ptr[0] = 0, row_ptr[n] = 2m as
  * stated by the caller, monotone offsets, ids < n, no self loop -- and a graph

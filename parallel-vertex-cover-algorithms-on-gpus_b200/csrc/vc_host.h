@@ -113,6 +113,7 @@ struct Ctx {
         int per_sm;
     };
     std::vector<Occ> occ;  // resident CTAs per SM, as asked for once per kernel and shared-memory size
+    std::mutex occ_mu;     // (a server is planned without `mu`)
     std::mutex mu;
 };
 

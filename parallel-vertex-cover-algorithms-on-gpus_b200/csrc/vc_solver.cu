@@ -267,6 +267,7 @@ static int ctas_per_sm(Ctx &c, F fn, uint32_t smem)
 {
     int per_sm = 0;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lk(c.occ_mu);
     for (const Ctx::Occ &o : c.occ)
         if (o.fn == (const void *)fn && o.smem == smem) return o.per_sm;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)NT, smem) != cudaSuccess) return 0;
