@@ -332,7 +332,8 @@ __device__ __forceinline__ void dense_restore(DSU<NW> &s, uint32_t pos)
 // A step is a chain of four ballots, two shuffles and two row loads, about a
 // hundred instructions, and a bound takes some forty of them: it is what a node
 // now spends most of its time on, bound by issue with the SM full and by that
-// chain's latency without.  It pays for itself many times over: 512 graphs of 30
+// chain's latency without.  (Two picks per step, and all vertices of degree 1 at
+// once, both made batches slower: 15.0 -> 16.8 and 15.3 -> 18.5 ms.)  It pays for itself many times over: 512 graphs of 30
 // to 160 vertices and average degree 3 to 12 in one batch take 1.6 M nodes and
 // 32 ms instead of 161 M and 470 ms; one of 197 vertices and 648 edges 16 k and
 // 1.6 ms instead of 3.6 M and 22 ms.  Degrees bit-sliced rather than in bytes
@@ -1147,12 +1148,12 @@ __device__ __forceinline__ void stage_graph(uint32_t *adj, const Params &P, uint
 
 // ---- first covers
 // A plain solve of a graph of 16 words or more whose average degree is at most 16
-// starts with dives on the first blocks after the one that takes up the search: the
-// last 913-vertex graph of a sparse pair went from 1.9 to 1.0 ms with its partner,
-// four graphs of 327..584 vertices from 4.6 to 3.5.  Dense graphs gain nothing; and
-// with smaller ones the nodes fall as much (175 vertices: 6,700 to 530) but not the
-// time (0.39 to 0.59 ms): against a tight incumbent a node's bound runs its full
-// course, and the chain of nodes to the first leaf is what such a tree's time is.
+// starts with dives on the first blocks after the one that takes up the search: two
+// graphs of 700 and 913 vertices and average degree 3.2 went from 1.9 to 1.0 ms, four
+// of 327..584 vertices from 4.6 to 3.5.  Dense graphs gain nothing; and with smaller
+// ones the nodes fall as much (175 vertices: 6,700 to 530) but not the time (0.39 to
+// 0.59 ms): against a tight incumbent a node's bound runs its full course, and the
+// chain of nodes to the first leaf is what such a tree's time is.
 constexpr uint32_t kDiveBlocks = 37;
 // One greedy dive: a vertex of least degree, at random among them, stays out of
 // the cover and its neighbours go in, until no edge is left.  The cover is left in
