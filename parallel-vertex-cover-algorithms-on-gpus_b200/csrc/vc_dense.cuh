@@ -333,12 +333,14 @@ __device__ __forceinline__ void dense_restore(DSU<NW> &s, uint32_t pos)
 // hundred instructions, and a bound takes some forty of them: it is what a node
 // now spends most of its time on, bound by issue with the SM full and by that
 // chain's latency without.  (Two picks per step, and all vertices of degree 1 at
-// once, both made batches slower: 15.0 -> 16.8 and 15.3 -> 18.5 ms.)  It pays for itself many times over: 512 graphs of 30
-// to 160 vertices and average degree 3 to 12 in one batch take 1.6 M nodes and
-// 32 ms instead of 161 M and 470 ms; one of 197 vertices and 648 edges 16 k and
-// 1.6 ms instead of 3.6 M and 22 ms.  Degrees bit-sliced rather than in bytes
-// (four to a word, a word per lane) took the 512 graphs from 66 to 49 ms, and
-// bounding both children of a node instead of each node as it is reached to 32.
+// once, both made batches slower: 15.0 -> 16.8 and 15.3 -> 18.5 ms.)  It pays for
+// itself many times over: 512 graphs of 30 to 160 vertices and average degree 3 to
+// 12 in one batch take 1.6 M nodes and 15.3 ms instead of 161 M and 470 ms; one of
+// 197 vertices and 648 edges 30 k and 0.88 ms instead of 3.6 M and 22 ms.  When the
+// bound went in, bit-slicing the degrees rather than holding them in bytes (four to
+// a word, a word per lane) took the 512 graphs from 66 to 49 ms, and bounding both
+// children of a node instead of each node as it is reached to 32; the rest came with
+// the launch shapes and the hand-over of work.
 constexpr int kPackPlanes = 5;  // degrees below 32
 constexpr uint32_t kPackNow = 1u << 31;  // beside InstState's flags in a unit's copy: the bound's time has come
 
