@@ -123,7 +123,8 @@ struct ReduceHead {
     uint32_t taken;        // vertices taken into the cover
     uint32_t last_pass;
     uint32_t bad;          // the CSR check failed: nothing was reduced
-    uint32_t pad[2];
+    uint32_t uneven;       // rows and degrees part (edges in one direction only): the rest is no graph
+    uint32_t pad;
 };
 
 // A graph to reduce at its root (csrc/vc_reduce.cu) and what is left of it.

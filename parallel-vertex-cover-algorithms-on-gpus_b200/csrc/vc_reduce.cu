@@ -11,7 +11,11 @@
 // cooperative launch, two grid barriers per pass; what is left is written out as
 // a graph of its own, rows in the old order, and goes to the kernel for its size
 // (csrc/vc_solver.cu).  The optimum is the number of vertices taken here plus the
-// rest's.
+// rest's.  A caller's device memory has been checked for its layout only: where an
+// edge is in one direction alone, a degree and the entries that are left of its row
+// can part.  The write-out keeps to the entries whose vertex is left and to the row's
+// own places, and a row that it does not fill exactly marks the graph as uneven:
+// its rest is not searched, the graph itself is.
 //
 // A pass decides the degree-one, degree-two/triangle and high-degree rules from
 // one snapshot, as the search units do (vc_search.cuh, reduce_pass; the
@@ -226,9 +230,9 @@ __global__ void __launch_bounds__(kReduceThreads, 2) k_reduce(ReduceArgs A)
             tc += s_cnt[w];
             ts += s_sum[w];
         }
+        const uint32_t id = base_c + wc + pc - 1u;
+        if (v < hi) __stcg(&A.map[v], d > 0u ? id : kNone);
         if (d > 0u) {
-            const uint32_t id = base_c + wc + pc - 1u;
-            __stcg(&A.map[v], id);
             __stcg(&A.inv[id], v);
             __stcg(&A.rrp[id], base_s + wsum + ps - d);
         }
@@ -237,19 +241,21 @@ __global__ void __launch_bounds__(kReduceThreads, 2) k_reduce(ReduceArgs A)
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) A.rrp[H->n] = H->m2;
     grid.sync();
-    // a warp per row that is left, its live entries in the old order
+    // a warp per row that is left, its entries that are left in the old order
     const uint32_t rows = __ldcg(&H->n);
     for (uint32_t id = t0 >> 5; id < rows; id += step >> 5) {
         const uint32_t v = __ldcg(&A.inv[id]);
         uint32_t out = __ldcg(&A.rrp[id]);
+        const uint32_t end = __ldcg(&A.rrp[id + 1]);
         const uint32_t e1 = __ldg(&A.rp[v + 1]);
         for (uint32_t eb = __ldg(&A.rp[v]); eb < e1; eb += 32) {
-            const uint32_t u = eb + lane < e1 ? __ldg(&A.cl[eb + lane]) : kNone;
-            const bool in = u != kNone && __ldcg(&A.taken[u]) == 0u;
-            const uint32_t m = __ballot_sync(0xffffffffu, in);
-            if (in) A.rcl[out + __popc(m & ((1u << lane) - 1u))] = __ldcg(&A.map[u]);
+            const uint32_t x = eb + lane < e1 ? __ldcg(&A.map[__ldg(&A.cl[eb + lane])]) : kNone;
+            const uint32_t m = __ballot_sync(0xffffffffu, x != kNone);
+            const uint32_t at = out + __popc(m & ((1u << lane) - 1u));
+            if (x != kNone && at < end) A.rcl[at] = x;
             out += __popc(m);
         }
+        if (out != end && lane == 0) __stcg(&H->uneven, 1u);
     }
 }
 

@@ -984,8 +984,8 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
         r.bound = req->instance == VC_PVC ? std::min<uint32_t>(req->k, g->n) + 1 : init_best_for(req, g->n);
         red.push_back(r);
         const vc_status s = run_reductions(*c, red, job.check, stream, &reduce_ms);
-        if (s == VC_ERR_NOMEM) {
-            red.clear();  // no room for it: the search reduces the root itself
+        if (s == VC_ERR_NOMEM || (s == VC_OK && red[0].h.uneven)) {
+            red.clear();  // no room for it, or no graph: the search reduces the root itself
         } else {
             const bool bad = s == VC_OK && red[0].h.bad;
             if (s != VC_OK || bad) {
@@ -1140,7 +1140,8 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         }
     }
     std::vector<const Reduce *> red_at(count, nullptr);
-    for (size_t j = 0; j < reds.size(); ++j) red_at[red_of[j]] = &reds[j];
+    for (size_t j = 0; j < reds.size(); ++j)
+        if (!reds[j].h.uneven) red_at[red_of[j]] = &reds[j];
     if (check == 2)
         for (const Reduce &r : reds)
             if (r.h.bad) return fail(VC_ERR_INVALID);
@@ -1166,6 +1167,10 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
     for (size_t j = 0; j < reds.size(); ++j) {
         const uint32_t i = red_of[j];
         Reduce &r = reds[j];
+        if (r.h.uneven) {  // searched as it is
+            searched[j] = 1;
+            continue;
+        }
         early[j] = out[i];
         if (r.h.bad) {  // device-resident input: this graph only
             early[j].cover_mask = nullptr;
