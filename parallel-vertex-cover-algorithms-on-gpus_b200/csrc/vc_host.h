@@ -127,15 +127,23 @@ struct ReduceHead {
     uint32_t pad;
 };
 
-// A graph to reduce at its root (csrc/vc_reduce.cu) and what is left of it.
-struct Reduce {
-    const uint32_t *rp = nullptr, *cl = nullptr;  // the graph
-    uint32_t n = 0, m2 = 0, bound = 0;
-    int32_t *deg = nullptr;  // device scratch and results
-    uint32_t *taken = nullptr, *map = nullptr, *inv = nullptr, *rrp = nullptr, *rcl = nullptr, *part = nullptr;
-    uint8_t *cover = nullptr;
+// What the reduction of a graph's root (csrc/vc_reduce.cu) reads and leaves.
+struct ReduceArgs {
+    const uint32_t *rp = nullptr, *cl = nullptr;
+    uint32_t n = 0, bound = 0;                   // high-degree rule: deg + taken >= bound
+    int32_t *deg = nullptr;
+    uint32_t *taken = nullptr;                   // the pass that took a vertex, 0 = live
+    uint32_t *map = nullptr, *inv = nullptr;     // old id -> new id, new id -> old id
+    uint32_t *rrp = nullptr, *rcl = nullptr;     // what is left
+    uint8_t *cover = nullptr;                    // 1 = taken
+    uint32_t *part = nullptr;                    // per CTA: vertices left, entries left
     ReduceHead *head = nullptr;
-    ReduceHead h = {};                // host copies
+};
+
+// A graph to reduce at its root, and the host's copies of what came of it.
+struct Reduce : ReduceArgs {
+    uint32_t m2 = 0;
+    ReduceHead h = {};
     const uint8_t *h_cover = nullptr;
     uint32_t *h_inv = nullptr;
 };
@@ -207,7 +215,8 @@ struct PlanOpts {
 Ctx *get_ctx(int dev, vc_status *err);
 cudaError_t make_plan(Ctx &c, uint32_t np, uint32_t nmax, Plan &pl, const PlanOpts &o = PlanOpts());
 void cap_plan(const Ctx &c, Plan &pl, uint32_t per_sm);
-cudaError_t launch_reduce(const Reduce &r, uint32_t ctas, cudaStream_t stream);
+cudaError_t launch_reduce(const ReduceArgs &r, uint32_t ctas, cudaStream_t stream);
+cudaError_t launch_reduce_many(const ReduceArgs *list, uint32_t count, uint32_t ctas, cudaStream_t stream);
 uint32_t reduce_ctas(const Ctx &c);
 vc_status run_job(Ctx &c, Job &job, cudaStream_t stream);
 vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_t n, vc_result *out);

@@ -749,82 +749,140 @@ vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_
 }
 
 // ---------------------------------------------------------------- large graphs
-// Checks and reduces the graphs at their roots; the answers come back in their
-// heads and covers (one synchronisation).  `arena` says where their scratch is:
-// offsets of the rests' rows are taken from its start.
-static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, cudaStream_t stream, float *ms)
+// How large graphs (largest first) are reduced.  Power-law graphs, measured one at a
+// time (kernel, us; a pass takes the same share of each):
+//   vertices            10,000   30,000   100,000
+//   whole chip             147      178       220
+//   cluster of 8 CTAs      250      503      1330
+//   cluster of 4           340      770      2310
+//   cluster of 2           550     1400      4510
+//   one CTA                955     2570      8520
+// that is 110 us and 46 more for every 512 vertices per CTA; but 37 clusters of 8 (or
+// 296 single CTAs) run side by side, and launches that take the chip one after another.
+// The first `chip` graphs get the chip and the others a cluster each, in the way that
+// these figures make cheapest.  1000 graphs of 1100 to 4000 vertices on the device,
+// planted and power-law: 1.4 and 1.9 ms a call, each with the chip in turn 69 and 125,
+// reduced by the search's own units 2.4 and 2.4; one of 100,000 beside 256 of them
+// 0.65, 17 and 12.
+struct ReduceSplit {
+    uint32_t chip, ctas;  // graphs that get the whole chip; CTAs per cluster for the others
+};
+static ReduceSplit split_reductions(const std::vector<Reduce> &reds, uint32_t resident)
+{
+    const uint32_t count = (uint32_t)reds.size();
+    ReduceSplit best{count, 8};
+    if (count == 1) return best;
+    const double chip = 160.0;
+    double sum[4] = {0, 0, 0, 0}, least = chip * count;
+    for (uint32_t k = count; k-- > 0;)  // the first k get the chip
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t ctas = 1u << j;
+            const double one = 110.0 + 46.0 * reds[k].n / (512.0 * ctas);
+            sum[j] += one;
+            const double t = chip * k + std::max(one, sum[j] * ctas / resident);
+            if (t < least) { least = t; best = {k, ctas}; }
+        }
+    return best;
+}
+
+// Checks and reduces the graphs (largest first) at their roots; the answers come back
+// in their heads and covers (one synchronisation).  Their rows are in rp and cl.
+static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, const uint32_t *rp, const uint32_t *cl,
+                                cudaStream_t stream, float *ms)
 {
     const uint32_t count = (uint32_t)reds.size(), ctas = reduce_ctas(c);
-    size_t words = 0, host = 0;
+    const ReduceSplit split = split_reductions(reds, ctas);
+    size_t words = 0;
     auto take = [&](size_t n) {  // 16-byte pieces
         const size_t at = words;
         words += (n + 3) / 4 * 4;
         return at;
     };
-    const size_t heads = take(count * sizeof(ReduceHead) / 4), descs = take(count * sizeof(InstDesc) / 4);
-    std::vector<size_t> at;
+    // one piece that goes in, one that comes back (the new ids only where there is a
+    // search to follow), and scratch
+    const size_t descs = take(count * sizeof(InstDesc) / 4), list = take(count * sizeof(ReduceArgs) / 4), in_words = words;
+    const size_t heads = take(count * sizeof(ReduceHead) / 4);
+    std::vector<size_t> cover_at, inv_at, at;
+    for (const Reduce &r : reds) cover_at.push_back(take((r.n + 3) / 4));
+    const size_t back_words = words - heads;
+    for (const Reduce &r : reds) inv_at.push_back(take(r.n));
+    const size_t pinned = words;
     for (const Reduce &r : reds) {
-        at.push_back(take(5ull * r.n + 1 + 2ull * ctas));
+        at.push_back(take(4ull * r.n + 1 + 2ull * ctas));
         at.push_back(take(r.m2));
-        at.push_back(take((r.n + 3) / 4));
     }
-    if (c.red.ensure(4 * words)) return VC_ERR_NOMEM;
-    uint32_t *base = (uint32_t *)c.red.p;
-    for (const Reduce &r : reds) host += (r.n + 15) / 16 * 16 + 4ull * r.n;
-    host += count * (sizeof(ReduceHead) + sizeof(InstDesc)) + 64;
-    if (c.h_red.ensure(host)) return VC_ERR_NOMEM;
-    uint8_t *h = (uint8_t *)c.h_red.p;
-    InstDesc *h_desc = (InstDesc *)h;
-    ReduceHead *h_head = (ReduceHead *)(h_desc + count);
-    uint8_t *h_at = (uint8_t *)(((uintptr_t)(h_head + count) + 15) & ~(uintptr_t)15);
+    if (c.red.ensure(4 * words) || c.h_red.ensure(4 * pinned)) return VC_ERR_NOMEM;
+    uint32_t *base = (uint32_t *)c.red.p, *h = (uint32_t *)c.h_red.p;
+    InstDesc *h_desc = (InstDesc *)(h + descs);
+    ReduceArgs *h_list = (ReduceArgs *)(h + list);
+    ReduceHead *d_head = (ReduceHead *)(base + heads), *h_head = (ReduceHead *)(h + heads);
     for (uint32_t i = 0; i < count; ++i) {
         Reduce &r = reds[i];
-        uint32_t *p = base + at[3 * i];
+        uint32_t *p = base + at[2 * i];
         r.deg = (int32_t *)p;
         r.taken = p + r.n;
         r.map = p + 2ull * r.n;
-        r.inv = p + 3ull * r.n;
-        r.rrp = p + 4ull * r.n;
-        r.part = p + 5ull * r.n + 1;
-        r.rcl = base + at[3 * i + 1];
-        r.cover = (uint8_t *)(base + at[3 * i + 2]);
-        r.head = (ReduceHead *)(base + heads) + i;
+        r.rrp = p + 3ull * r.n;
+        r.part = p + 4ull * r.n + 1;
+        r.rcl = base + at[2 * i + 1];
+        r.inv = base + inv_at[i];
+        r.cover = (uint8_t *)(base + cover_at[i]);
+        r.head = d_head + i;
+        r.h_inv = h + inv_at[i];
+        r.h_cover = (const uint8_t *)(h + cover_at[i]);
+        h_list[i] = r;
         InstDesc d{};
         d.n = r.n;
         d.m2 = r.m2;
+        d.row_off = (uint64_t)(r.rp - rp);
+        d.col_off = (uint64_t)(r.cl - cl);
         h_desc[i] = d;
-        r.h_inv = (uint32_t *)h_at;
-        h_at += 4ull * r.n;
-        r.h_cover = h_at;
-        h_at += (r.n + 15) / 16 * 16;
     }
-    const InstDesc *d_desc = (const InstDesc *)(base + descs);
-    bool ok = cudaMemsetAsync(base + heads, 0, count * sizeof(ReduceHead), stream) == cudaSuccess &&
-              cudaMemcpyAsync(base + descs, h_desc, count * sizeof(InstDesc), cudaMemcpyHostToDevice, stream) == cudaSuccess;
+    bool ok = cudaMemsetAsync(d_head, 0, count * sizeof(ReduceHead), stream) == cudaSuccess &&
+              cudaMemcpyAsync(base, h, 4 * in_words, cudaMemcpyHostToDevice, stream) == cudaSuccess;
     cudaEventRecord(c.ev0, stream);
-    for (uint32_t i = 0; ok && i < count; ++i) {
-        const Reduce &r = reds[i];
-        if (check) {
-            ok = launch_check(check == 2, r.rp, r.cl, d_desc + i, &r.head->bad, 1, 1u, 1, r.n, stream) == cudaSuccess;
-            g_launches += 1;
-        }
-        ok = ok && launch_reduce(r, ctas, stream) == cudaSuccess;
+    auto check_from = [&](uint32_t i, uint32_t k, uint32_t nmax) {  // graphs i .. i + k - 1 of the list
+        if (!check || k == 0) return;
+        ok = ok && launch_check(check == 2, rp, cl, (const InstDesc *)(base + descs) + i, &d_head[i].bad,
+                                sizeof(ReduceHead) / 4, 1u, k, nmax, stream) == cudaSuccess;
         g_launches += 1;
-        ok = ok && cudaMemcpyAsync((void *)r.h_cover, r.cover, r.n, cudaMemcpyDeviceToHost, stream) == cudaSuccess;
+    };
+    for (uint32_t i = 0; i < split.chip; ++i) check_from(i, 1, reds[i].n);  // a launch's blocks are as many for each of its graphs
+    if (split.chip < count) check_from(split.chip, count - split.chip, reds[split.chip].n);
+    for (uint32_t i = 0; ok && i < split.chip; ++i) {
+        ok = launch_reduce(reds[i], ctas, stream) == cudaSuccess;
+        g_launches += 1;
+    }
+    if (split.chip < count) {
+        ok = ok && launch_reduce_many((const ReduceArgs *)(base + list) + split.chip, count - split.chip, split.ctas, stream) == cudaSuccess;
+        g_launches += 1;
     }
     cudaEventRecord(c.ev1, stream);
-    ok = ok && cudaMemcpyAsync(h_head, base + heads, count * sizeof(ReduceHead), cudaMemcpyDeviceToHost, stream) == cudaSuccess;
+    ok = ok && cudaMemcpyAsync(h_head, d_head, 4 * back_words, cudaMemcpyDeviceToHost, stream) == cudaSuccess;
     if (cudaStreamSynchronize(stream) != cudaSuccess || !ok) return VC_ERR_CUDA;
     cudaEventElapsedTime(ms, c.ev0, c.ev1);
     for (uint32_t i = 0; i < count; ++i) reds[i].h = h_head[i];
     Plan pl;  // what vc_debug_stats reports if there is nothing left to search
     pl.block = 512;
-    pl.grid = std::min<uint32_t>((reds.back().n + pl.block - 1) / pl.block, ctas);
-    pl.np = (reds.back().n + 31) / 32 * 32;
+    pl.grid = std::min<uint32_t>((reds[0].n + pl.block - 1) / pl.block, ctas);
+    pl.np = (reds[0].n + 31) / 32 * 32;
     c.last_plan = pl;
     c.last_num_su = 0;
     c.last_stats.clear();
     return VC_OK;
+}
+
+// The new ids of the rests that are searched, for fill_result (part of the next
+// synchronisation): a copy each, or one of all where they are many.
+static void fetch_new_ids(const std::vector<Reduce> &reds, const std::vector<uint8_t> &searched, cudaStream_t stream)
+{
+    if (std::count(searched.begin(), searched.end(), 1) > 8) {
+        const Reduce &a = reds.front(), &z = reds.back();
+        cudaMemcpyAsync(a.h_inv, a.inv, 4ull * (z.inv - a.inv + z.n), cudaMemcpyDeviceToHost, stream);
+        return;
+    }
+    for (size_t j = 0; j < reds.size(); ++j)
+        if (searched[j]) cudaMemcpyAsync(reds[j].h_inv, reds[j].inv, 4ull * reds[j].h.n, cudaMemcpyDeviceToHost, stream);
 }
 
 // The search a reduction leaves to do: false if there is none (out's answer is
@@ -983,7 +1041,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
         r.m2 = 2 * g->m;
         r.bound = req->instance == VC_PVC ? std::min<uint32_t>(req->k, g->n) + 1 : init_best_for(req, g->n);
         red.push_back(r);
-        const vc_status s = run_reductions(*c, red, job.check, stream, &reduce_ms);
+        const vc_status s = run_reductions(*c, red, job.check, r.rp, r.cl, stream, &reduce_ms);
         if (s == VC_ERR_NOMEM || (s == VC_OK && red[0].h.uneven)) {
             red.clear();  // no room for it, or no graph: the search reduces the root itself
         } else {
@@ -1002,7 +1060,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
             job.d_col = red[0].rcl;
             job.check = 0;
             job.rest.push_back(&red[0]);
-            cudaMemcpyAsync(red[0].h_inv, red[0].inv, 4ull * d.n, cudaMemcpyDeviceToHost, stream);
+            fetch_new_ids(red, {1}, stream);
             job.wide = d.n <= kWideMaxN && red[0].h.maxd <= 254;
         }
     }
@@ -1108,13 +1166,15 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
     }
     const int check = d_rp ? 1 : (on_device ? 2 : 0);
     float total_kernel = 0;
-    // Large graphs first: each root is reduced by the whole chip, and the search
-    // gets what is left of it.
+    // Large graphs first: their roots are reduced (largest first) and the search gets
+    // what is left of them.
     std::vector<Reduce> reds;
     std::vector<uint32_t> red_of;  // the graph each reduction is of
     if (!c->force_sparse) {
-        for (uint32_t i = 0; i < count; ++i) {
-            if (a->n[i] <= kHalfMaxN) continue;
+        for (uint32_t i = 0; i < count; ++i)
+            if (a->n[i] > kHalfMaxN) red_of.push_back(i);
+        std::stable_sort(red_of.begin(), red_of.end(), [&](uint32_t x, uint32_t y) { return a->n[x] > a->n[y]; });
+        for (const uint32_t i : red_of) {
             const uint32_t *rp = a->row_ptr + a->row_off[i];
             Reduce r;
             r.rp = job.d_rp + a->row_off[i];
@@ -1123,7 +1183,6 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
             r.m2 = rp[r.n];
             r.bound = reqs[i].instance == VC_PVC ? std::min<uint32_t>(reqs[i].k, r.n) + 1 : init_best_for(&reqs[i], r.n);
             reds.push_back(r);
-            red_of.push_back(i);
         }
     }
     struct Trim {
@@ -1131,7 +1190,7 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         ~Trim() { trim_reductions(*c); }
     } trim{c};
     if (!reds.empty()) {
-        const vc_status s = run_reductions(*c, reds, check, stream, &total_kernel);
+        const vc_status s = run_reductions(*c, reds, check, job.d_rp, job.d_col, stream, &total_kernel);
         if (s == VC_ERR_NOMEM) {
             reds.clear();  // no room: the search reduces the roots itself
             red_of.clear();
@@ -1184,9 +1243,9 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         early[j].cover_mask = nullptr;  // written below, when every launch has gone well
         if (!rest_of(r, &reqs[i], total_kernel, rest[j], &early[j])) continue;
         searched[j] = 1;
-        cudaMemcpyAsync(r.h_inv, r.inv, 4ull * rest[j].n, cudaMemcpyDeviceToHost, stream);
         cls[i] = 5 + klass(rest[j].n, rest[j].n <= kWideMaxN && r.h.maxd <= 254);
     }
+    fetch_new_ids(reds, searched, stream);
     for (uint32_t i = 0; i < count; ++i)
         if (a->n[i] > 0 && !red_at[i]) cls[i] = klass(a->n[i], wide_ok(a->n[i], a->row_ptr + a->row_off[i]));
     std::vector<Job> jobs;
