@@ -1346,7 +1346,7 @@ __device__ bool acquire_cta(DSU<NW> &s, const Params &P, CtaPool &cp, uint32_t *
                         atomicExch(&cp.hdr[kCpExit], 1u);
                         res = 3;
                     } else if (globaltimer() > s.deadline) {
-                        atomicExch(&P.ctl[kAbort], 1ull);
+                        stop_launch(P, kStopTime);
                         atomicExch(&cp.hdr[kCpExit], 1u);
                         res = 3;
                     }
@@ -1492,7 +1492,7 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
                 w = ld_relaxed_u64(&P.ctl[kState]);
                 if ((ticks & 255u) == 0u) {
                     if (ld_relaxed_u64(&P.ctl[kAbort])) f |= kError;
-                    else if (globaltimer() > s.deadline) { atomicExch(&P.ctl[kAbort], 1ull); f |= kError; }
+                    else if (globaltimer() > s.deadline) { stop_launch(P, kStopTime); f |= kError; }
                 }
                 if (!packing && globaltimer() > t_pack) f |= kPackNow;
             }

@@ -160,7 +160,7 @@ struct Job {
     std::vector<uint32_t> covers;
     float kernel_ms = 0;
     unsigned long long t0 = 0;
-    bool aborted = false;
+    unsigned long long stopped = 0;  // the control word kAbort
     bool wide = false;  // every graph may take the 20-word dense kernel
     bool half = false;  // every graph may take the 16/32-word dense kernels (16-bit degrees)
     int check = 0;  // k_check_csr before the search: 0 none, 1 the layout (caller's device memory), 2 all of it
@@ -211,6 +211,9 @@ struct PlanOpts {
     bool lane = false;         // a server lane, which shares the SMs with other lanes' kernels
     const Tune *tune = nullptr; // the size class's tuned shape, if any
 };
+
+// The status of a graph whose search a launch left unfinished (its control word kAbort).
+inline vc_status stopped_status(unsigned long long why) { return why == vcg::kStopTime ? VC_TIMEOUT : VC_ERR_INTERNAL; }
 
 Ctx *get_ctx(int dev, vc_status *err);
 cudaError_t make_plan(Ctx &c, uint32_t np, uint32_t nmax, Plan &pl, const PlanOpts &o = PlanOpts());

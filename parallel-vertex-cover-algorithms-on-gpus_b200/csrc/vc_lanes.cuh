@@ -612,7 +612,7 @@ __device__ void lanes_main(const Params &P, uint32_t *sm, uint32_t *hdr)
                 if (vld(&hdr[kLhExit])) {
                     res = 3;
                 } else if (globaltimer() > deadline) {
-                    atomicExch(&P.ctl[kAbort], 1ull);
+                    stop_launch(P, kStopTime);
                     atomicExch(&hdr[kLhExit], 1u);
                     res = 3;
                 } else if (vld(&hdr[kLhCount]) > 0) {
@@ -781,7 +781,7 @@ __device__ void lanes_main(const Params &P, uint32_t *sm, uint32_t *hdr)
                 w = ld_relaxed_u64(&P.ctl[kState]);
                 if ((it & 255u) == 0u) {
                     if (ld_relaxed_u64(&P.ctl[kAbort])) aborted = kError;
-                    else if (globaltimer() > deadline) { atomicExch(&P.ctl[kAbort], 1ull); aborted = kError; }
+                    else if (globaltimer() > deadline) { stop_launch(P, kStopTime); aborted = kError; }
                 }
                 f |= aborted;
             }

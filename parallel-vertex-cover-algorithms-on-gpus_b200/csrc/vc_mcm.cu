@@ -156,7 +156,7 @@ __device__ __forceinline__ bool mcm_acquire(const Params &P, const McmArgs &A, I
                 atomicAdd(&P.ctl[kState], 0xfffffffeffffffffull);  // pending - 1, idle units - 1
                 res = 1;
             } else if (globaltimer() > deadline) {
-                atomicExch(&P.ctl[kAbort], 1ull);
+                stop_launch(P, kStopTime);
                 res = 2;
             }
         }
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
                 w = ld_relaxed_u64(&P.ctl[kState]);
                 if ((ticks & 255u) == 0u) {
                     if (ld_relaxed_u64(&P.ctl[kAbort])) f |= kError;
-                    else if (globaltimer() > deadline) { atomicExch(&P.ctl[kAbort], 1ull); f |= kError; }
+                    else if (globaltimer() > deadline) { stop_launch(P, kStopTime); f |= kError; }
                 }
             }
             c_best = __shfl_sync(0xffffffffu, b, 0);
@@ -451,7 +451,8 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
     out->kernel_ms = ms;
     if (s1.flags & kFound) out->status = VC_OK;  // every vertex matched or isolated: nothing can exceed it
     else if (s1.flags & kBudget) out->status = VC_BUDGET;
-    else if (abort_word || (s1.flags & kError)) out->status = VC_TIMEOUT;
+    else if (abort_word) out->status = stopped_status(abort_word);
+    else if (s1.flags & kError) out->status = VC_TIMEOUT;
     else out->status = VC_OK;
     out->total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return out->status;

@@ -111,7 +111,7 @@ __global__ void k_noalloc_finish(const Scratch *s, uint32_t ub, uint32_t *result
     if (st.flags & kBadGraph) status = VC_ERR_INVALID;
     else if (st.flags & kError) status = VC_ERR_INTERNAL;
     else if (st.flags & kBudget) status = VC_BUDGET;
-    else if ((st.flags & kCut) || !(st.flags & kDone)) status = s->ctl[kAbort] ? VC_TIMEOUT : VC_ERR_INTERNAL;
+    else if ((st.flags & kCut) || !(st.flags & kDone)) status = s->ctl[kAbort] == kStopTime ? VC_TIMEOUT : VC_ERR_INTERNAL;
     else status = VC_OK;
     uint32_t size, decision;
     if (d.mode == kModeMVC) {

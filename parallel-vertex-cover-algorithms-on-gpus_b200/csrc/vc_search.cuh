@@ -678,6 +678,9 @@ __device__ __forceinline__ void load_root(SU &s)
     G::sync();
 }
 
+// Every unit gives up its work as soon as it sees the word.
+__device__ __forceinline__ void stop_launch(const Params &P, unsigned long long why) { atomicMax(&P.ctl[kAbort], why); }
+
 // ---------------------------------------------------------------- global ring
 // Bounded MPMC ring.  Places are handed out by fetch-and-add tickets, to a
 // producer against the pending count and to a consumer against the count of
@@ -693,9 +696,10 @@ __device__ __forceinline__ bool ring_wait(const Params &P, unsigned long long po
 {
     for (int it = 0; it < kRingSpins; ++it) {
         if (ld_acquire_u64(&P.pool_seq[pos & P.q_mask]) == seq) return true;
+        if ((it & 255) == 255 && ld_relaxed_u64(&P.ctl[kAbort])) return false;
         __nanosleep(32);
     }
-    atomicExch(&P.ctl[kAbort], 1ull);
+    stop_launch(P, kStopRing);
     return false;
 }
 
@@ -1070,7 +1074,7 @@ __device__ bool acquire(S &s, const Params &P, CtaPool &cp, bool &cursor_open)
                         atomicExch(&cp.hdr[kCpExit], 1u);
                         res = 3;
                     } else if (globaltimer() > s.deadline) {
-                        atomicExch(&P.ctl[kAbort], 1ull);
+                        stop_launch(P, kStopTime);
                         atomicExch(&cp.hdr[kCpExit], 1u);
                         res = 3;
                     }
@@ -1178,7 +1182,7 @@ __device__ void su_main(const Params &P, uint8_t *ws, CtaPool &cp)
                 w = ld_relaxed_u64(&P.ctl[kState]);
                 if ((ticks & 255u) == 0u) {
                     if (ld_relaxed_u64(&P.ctl[kAbort])) f |= kError;
-                    else if (globaltimer() > s.deadline) { atomicExch(&P.ctl[kAbort], 1ull); f |= kError; }
+                    else if (globaltimer() > s.deadline) { stop_launch(P, kStopTime); f |= kError; }
                 }
             }
             s.c_best = G::bcast(b);

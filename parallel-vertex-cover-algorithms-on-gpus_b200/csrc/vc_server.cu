@@ -389,7 +389,7 @@ uint32_t collect(SrvLane *s)
     return got;
 }
 
-// After an abnormal kernel exit, requests still in flight get a timeout status.
+// After an abnormal kernel exit, requests still in flight get its status.
 void fail_inflight(SrvLane *s, vc_status st)
 {
     s->discard_queue = true;
@@ -430,7 +430,8 @@ void request_loop(SrvLane *s)
             collect(s);
             unsigned long long abort_flag = 0;
             cudaMemcpy(&abort_flag, (unsigned long long *)s->ctl.p + kAbort, sizeof(abort_flag), cudaMemcpyDeviceToHost);
-            if (abort_flag || cudaGetLastError() != cudaSuccess) fail_inflight(s, VC_TIMEOUT);
+            const bool failed = cudaGetLastError() != cudaSuccess;
+            if (abort_flag || failed) fail_inflight(s, abort_flag ? stopped_status(abort_flag) : VC_TIMEOUT);
             progress = true;
         }
         if (!s->stop) {

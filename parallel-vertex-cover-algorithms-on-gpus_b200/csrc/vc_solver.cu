@@ -675,7 +675,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     const unsigned long long *h_ctl = (const unsigned long long *)h_out;
     job.t0 = h_ctl[kT0];
     cudaEventElapsedTime(&job.kernel_ms, c.ev0, c.ev1);
-    job.aborted = h_ctl[kAbort] != 0;
+    job.stopped = h_ctl[kAbort];
     job.st.assign((const InstState *)(h_out + st_at), (const InstState *)(h_out + st_at) + count);
     job.covers.assign((const uint32_t *)(h_out + covers_at), (const uint32_t *)(h_out + covers_at) + cover_words);
     job.plan = pl;
@@ -728,7 +728,7 @@ vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_
     if (s.flags & kBadGraph) st = VC_ERR_INVALID;
     else if (s.flags & kError) st = VC_ERR_INTERNAL;
     else if (s.flags & kBudget) st = VC_BUDGET;
-    else if ((s.flags & kCut) || !(s.flags & kDone)) st = job.aborted ? VC_TIMEOUT : VC_ERR_INTERNAL;
+    else if ((s.flags & kCut) || !(s.flags & kDone)) st = stopped_status(job.stopped);
     else st = VC_OK;
     out->status = st;
     out->tree_nodes = s.nodes;

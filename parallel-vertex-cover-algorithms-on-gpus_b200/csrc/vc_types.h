@@ -34,6 +34,12 @@ enum : uint32_t {
     kCtlWords = 192
 };
 
+// control word kAbort: why the launch stopped before its end (the largest counts)
+enum : unsigned long long {
+    kStopTime = 1,  // its time limit
+    kStopRing = 2,  // a wait on the ring ran out: a fault of the search, not the caller's limit
+};
+
 enum : uint32_t { kModeMVC = 0, kModePVC = 1 };
 
 // Per-SU counters (the role of the reference's Counters.cuh phase timers and
