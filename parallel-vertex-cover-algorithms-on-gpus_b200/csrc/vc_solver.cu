@@ -1004,7 +1004,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
         out->total_ms = 0;
         return VC_OK;
     }
-    if (g->n > kMaxVertices) return VC_ERR_TOO_LARGE;
+    if (g->n > kMaxVertices) return on_device && validate_csr(g) != VC_OK ? VC_ERR_INVALID : VC_ERR_TOO_LARGE;
     vc_status err;
     Ctx *c = get_ctx(req->device, &err);
     if (!c) return on_device && validate_csr(g) != VC_OK ? VC_ERR_INVALID : err;
