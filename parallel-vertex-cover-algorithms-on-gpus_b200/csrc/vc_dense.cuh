@@ -1454,7 +1454,8 @@ __device__ void su_main_dense(const Params &P, uint8_t *ws, uint32_t *adj, CtaPo
             if (lane == 0) cp.hdr[kCpStaged] = __ldcg(&P.inst[0].key);
         }
         __syncthreads();
-        if (!(G::bcast(ld_relaxed_u32(&P.st[0].flags)) & kBadGraph)) dive_on<NW>(s, P, 0);
+        const bool refused = (ld_relaxed_u32(&P.st[0].flags) & kBadGraph) || ld_relaxed_u64(&P.ctl[kAbort]) == kStopInput;
+        if (!G::bcast((uint32_t)refused)) dive_on<NW>(s, P, 0);
     }
 
     for (;;) {

@@ -122,7 +122,7 @@ struct ReduceHead {
     uint32_t n, m2, maxd;  // what is left: vertices, entries, largest degree
     uint32_t taken;        // vertices taken into the cover
     uint32_t last_pass;
-    uint32_t bad;          // the CSR check failed: nothing was reduced
+    uint32_t bad;          // the CSR check failed: nothing was reduced (a host-resident call: the first head's is for all)
     uint32_t uneven;       // rows and degrees part (edges in one direction only): the rest is no graph
     uint32_t pad;
 };
@@ -138,6 +138,7 @@ struct ReduceArgs {
     uint8_t *cover = nullptr;                    // 1 = taken
     uint32_t *part = nullptr;                    // per CTA: vertices left, entries left
     ReduceHead *head = nullptr;
+    const uint32_t *bad = nullptr;               // not 0: nothing is reduced
 };
 
 // A graph to reduce at its root, and the host's copies of what came of it.
@@ -163,7 +164,10 @@ struct Job {
     unsigned long long stopped = 0;  // the control word kAbort
     bool wide = false;  // every graph may take the 20-word dense kernel
     bool half = false;  // every graph may take the 16/32-word dense kernels (16-bit degrees)
-    int check = 0;  // k_check_csr before the search: 0 none, 1 the layout (caller's device memory), 2 all of it
+    // k_check_csr before the search: 0 none, 1 the layout (caller's device memory; a graph that fails is flagged), 2
+    // all of it (one that fails stops the launch: VC_ERR_INVALID), with 2 also of the graphs in `others`
+    int check = 0;
+    std::vector<vcg::InstDesc> others;
     std::vector<const Reduce *> rest;  // per graph: the reduction it is the rest of (empty: none are)
     const Tune *tune = nullptr;  // a shape to try instead of the context's table (the tuner's candidates)
     Plan plan;

@@ -91,7 +91,7 @@ __device__ __forceinline__ void reduce_graph(const ReduceArgs &A)
     const uint32_t t0 = cta * kReduceThreads + threadIdx.x, step = ctas * kReduceThreads;
     const uint32_t rounds = (A.n + step - 1) / step;  // the same for every thread: the warps stay whole
     vch::ReduceHead *H = A.head;
-    if (H->bad) return;  // the check before this launch: the same for every CTA
+    if (*A.bad) return;  // the check before this launch: the same for every CTA
     for (uint32_t v = t0; v < A.n; v += step) {
         A.deg[v] = (int32_t)(__ldg(&A.rp[v + 1]) - __ldg(&A.rp[v]));
         A.taken[v] = 0u;

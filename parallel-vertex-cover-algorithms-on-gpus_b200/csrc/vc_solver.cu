@@ -571,7 +571,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     size_t gws_bytes = pl.global_ws ? (size_t)pl.num_su * pl.su_bytes : 0;
     // One piece in (the descriptors, with a small host-resident graph) and one out
     // (control words, states, covers), each mirrored in pinned memory: one copy each.
-    const size_t rp_at = sizeof(InstDesc) * (size_t)count;
+    const size_t also_at = sizeof(InstDesc) * (size_t)count, rp_at = also_at + sizeof(InstDesc) * job.others.size();
     const size_t col_at = rp_at + (job.h_rp ? 4ull * (job.desc[0].n + 1) : 0);
     const size_t in_bytes = col_at + (job.h_rp ? 4ull * job.desc[0].m2 : 0);
     const size_t st_at = sizeof(unsigned long long) * kCtlWords, covers_at = st_at + sizeof(InstState) * (size_t)count;
@@ -600,6 +600,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     {
         uint8_t *h = (uint8_t *)c.h_in.p;
         memcpy(h, job.desc.data(), sizeof(InstDesc) * count);
+        memcpy(h + also_at, job.others.data(), rp_at - also_at);
         if (job.h_rp) {
             memcpy(h + rp_at, job.h_rp, col_at - rp_at);
             if (in_bytes > col_at) memcpy(h + col_at, job.h_col, in_bytes - col_at);
@@ -624,8 +625,12 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     if (launch_prepare(adj_words ? nw : 0, nmax, A, stream) != cudaSuccess) return VC_ERR_CUDA;
     g_launches += 1;
     if (job.check) {
-        if (launch_check(job.check == 2, job.d_rp, job.d_col, A.inst, &A.st->flags, sizeof(InstState) / 4, kBadGraph, count,
-                         nmax, stream) != cudaSuccess)
+        const bool all = job.check == 2;
+        uint32_t most = nmax;
+        for (const auto &d : job.others) most = std::max(most, d.n);
+        if (launch_check(all, job.d_rp, job.d_col, A.inst, all ? (uint32_t *)&A.ctl[kAbort] : &A.st->flags,
+                         all ? 0u : sizeof(InstState) / 4, all ? (uint32_t)kStopInput : kBadGraph,
+                         count + (uint32_t)job.others.size(), most, stream) != cudaSuccess)
             return VC_ERR_CUDA;
         g_launches += 1;
     }
@@ -676,6 +681,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     job.t0 = h_ctl[kT0];
     cudaEventElapsedTime(&job.kernel_ms, c.ev0, c.ev1);
     job.stopped = h_ctl[kAbort];
+    if (job.stopped == kStopInput) return VC_ERR_INVALID;
     job.st.assign((const InstState *)(h_out + st_at), (const InstState *)(h_out + st_at) + count);
     job.covers.assign((const uint32_t *)(h_out + covers_at), (const uint32_t *)(h_out + covers_at) + cover_words);
     job.plan = pl;
@@ -786,9 +792,11 @@ static ReduceSplit split_reductions(const std::vector<Reduce> &reds, uint32_t re
 }
 
 // Checks and reduces the graphs (largest first) at their roots; the answers come back
-// in their heads and covers (one synchronisation).  Their rows are in rp and cl.
+// in their heads and covers (one synchronisation).  Their rows are in rp and cl.  With
+// check 2 the call's other graphs are checked too, and one that fails stops every
+// reduction: VC_ERR_INVALID.
 static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, const uint32_t *rp, const uint32_t *cl,
-                                cudaStream_t stream, float *ms)
+                                const std::vector<InstDesc> &others, cudaStream_t stream, float *ms)
 {
     const uint32_t count = (uint32_t)reds.size(), ctas = reduce_ctas(c);
     const ReduceSplit split = split_reductions(reds, ctas);
@@ -800,7 +808,8 @@ static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, co
     };
     // one piece that goes in, one that comes back (the new ids only where there is a
     // search to follow), and scratch
-    const size_t descs = take(count * sizeof(InstDesc) / 4), list = take(count * sizeof(ReduceArgs) / 4), in_words = words;
+    const uint32_t checked = count + (check == 2 ? (uint32_t)others.size() : 0u);
+    const size_t descs = take(checked * sizeof(InstDesc) / 4), list = take(count * sizeof(ReduceArgs) / 4), in_words = words;
     const size_t heads = take(count * sizeof(ReduceHead) / 4);
     std::vector<size_t> cover_at, inv_at, at;
     for (const Reduce &r : reds) cover_at.push_back(take((r.n + 3) / 4));
@@ -828,6 +837,7 @@ static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, co
         r.inv = base + inv_at[i];
         r.cover = (uint8_t *)(base + cover_at[i]);
         r.head = d_head + i;
+        r.bad = &d_head[check == 2 ? 0 : i].bad;
         r.h_inv = h + inv_at[i];
         r.h_cover = (const uint8_t *)(h + cover_at[i]);
         h_list[i] = r;
@@ -838,17 +848,23 @@ static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, co
         d.col_off = (uint64_t)(r.cl - cl);
         h_desc[i] = d;
     }
+    uint32_t others_n = 0;
+    for (uint32_t i = count; i < checked; ++i) {
+        h_desc[i] = others[i - count];
+        others_n = std::max(others_n, h_desc[i].n);
+    }
     bool ok = cudaMemsetAsync(d_head, 0, count * sizeof(ReduceHead), stream) == cudaSuccess &&
               cudaMemcpyAsync(base, h, 4 * in_words, cudaMemcpyHostToDevice, stream) == cudaSuccess;
     cudaEventRecord(c.ev0, stream);
     auto check_from = [&](uint32_t i, uint32_t k, uint32_t nmax) {  // graphs i .. i + k - 1 of the list
         if (!check || k == 0) return;
-        ok = ok && launch_check(check == 2, rp, cl, (const InstDesc *)(base + descs) + i, &d_head[i].bad,
-                                sizeof(ReduceHead) / 4, 1u, k, nmax, stream) == cudaSuccess;
+        ok = ok && launch_check(check == 2, rp, cl, (const InstDesc *)(base + descs) + i, &d_head[check == 2 ? 0 : i].bad,
+                                check == 2 ? 0u : sizeof(ReduceHead) / 4, 1u, k, nmax, stream) == cudaSuccess;
         g_launches += 1;
     };
     for (uint32_t i = 0; i < split.chip; ++i) check_from(i, 1, reds[i].n);  // a launch's blocks are as many for each of its graphs
     if (split.chip < count) check_from(split.chip, count - split.chip, reds[split.chip].n);
+    check_from(count, checked - count, others_n);
     for (uint32_t i = 0; ok && i < split.chip; ++i) {
         ok = launch_reduce(reds[i], ctas, stream) == cudaSuccess;
         g_launches += 1;
@@ -869,7 +885,7 @@ static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, co
     c.last_plan = pl;
     c.last_num_su = 0;
     c.last_stats.clear();
-    return VC_OK;
+    return check == 2 && h_head[0].bad ? VC_ERR_INVALID : VC_OK;
 }
 
 // The new ids of the rests that are searched, for fill_result (part of the next
@@ -1041,7 +1057,7 @@ extern "C" vc_status vc_solve(const vc_csr *g, const vc_request *req, vc_result 
         r.m2 = 2 * g->m;
         r.bound = req->instance == VC_PVC ? std::min<uint32_t>(req->k, g->n) + 1 : init_best_for(req, g->n);
         red.push_back(r);
-        const vc_status s = run_reductions(*c, red, job.check, r.rp, r.cl, stream, &reduce_ms);
+        const vc_status s = run_reductions(*c, red, job.check, r.rp, r.cl, {}, stream, &reduce_ms);
         if (s == VC_ERR_NOMEM || (s == VC_OK && red[0].h.uneven)) {
             red.clear();  // no room for it, or no graph: the search reduces the root itself
         } else {
@@ -1164,8 +1180,22 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         job.d_rp = (const uint32_t *)c->rp.p;
         job.d_col = (const uint32_t *)c->col.p;
     }
-    const int check = d_rp ? 1 : (on_device ? 2 : 0);
+    int check = d_rp ? 1 : (on_device ? 2 : 0);
     float total_kernel = 0;
+    // graph i as the checks and the searches read it
+    auto desc_of = [&](uint32_t i) {
+        InstDesc d{};
+        d.n = a->n[i];
+        d.nw = (d.n + 31) / 32;
+        d.row_off = a->row_off[i];
+        d.col_off = a->col_off[i];
+        d.mode = reqs[i].instance == VC_PVC ? kModePVC : kModeMVC;
+        d.k = std::min<uint32_t>(reqs[i].k, d.n);
+        d.init_best = init_best_for(&reqs[i], d.n);
+        d.node_limit = reqs[i].node_limit;
+        d.m2 = a->row_ptr[a->row_off[i] + d.n];
+        return d;
+    };
     // Large graphs first: their roots are reduced (largest first) and the search gets
     // what is left of them.
     std::vector<Reduce> reds;
@@ -1190,20 +1220,22 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         ~Trim() { trim_reductions(*c); }
     } trim{c};
     if (!reds.empty()) {
-        const vc_status s = run_reductions(*c, reds, check, job.d_rp, job.d_col, stream, &total_kernel);
+        std::vector<InstDesc> others;
+        for (uint32_t i = 0; check == 2 && i < count; ++i)
+            if (a->n[i] > 0 && a->n[i] <= kHalfMaxN) others.push_back(desc_of(i));
+        const vc_status s = run_reductions(*c, reds, check, job.d_rp, job.d_col, others, stream, &total_kernel);
         if (s == VC_ERR_NOMEM) {
             reds.clear();  // no room: the search reduces the roots itself
             red_of.clear();
         } else if (s != VC_OK) {
             return fail(s);
+        } else if (check == 2) {
+            check = 0;  // every graph has passed
         }
     }
     std::vector<const Reduce *> red_at(count, nullptr);
     for (size_t j = 0; j < reds.size(); ++j)
         if (!reds[j].h.uneven) red_at[red_of[j]] = &reds[j];
-    if (check == 2)
-        for (const Reduce &r : reds)
-            if (r.h.bad) return fail(VC_ERR_INVALID);
     vc_status first = VC_OK;
     std::vector<vc_status> got(count, VC_OK);
     // One launch per kernel shape: dense bitsets (n <= 255), wide dense bitsets
@@ -1262,6 +1294,11 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
         cj.wide = cl % 5 == 1;
         cj.half = cl % 5 == 2;
         cj.check = rests ? 0 : check;
+        if (check == 2) {  // the first launch's checks are for the whole call: no graph is searched before all have passed
+            for (uint32_t i = 0; i < count; ++i)
+                if (cls[i] >= 0 && cls[i] != cl) cj.others.push_back(desc_of(i));
+            check = 0;
+        }
         cj.desc.resize(mem.size());
         double tl = 0;
         for (size_t j = 0; j < mem.size(); ++j) {
@@ -1274,24 +1311,14 @@ vc_status vc_solve_batch_impl(const vc_csr_arena *a, const vc_request *reqs, vc_
                 d.col_off = (uint64_t)(r->rcl - (const uint32_t *)c->red.p);
                 cj.rest.push_back(r);
             } else {
-                d.n = a->n[i];
-                d.nw = (d.n + 31) / 32;
-                d.row_off = a->row_off[i];
-                d.col_off = a->col_off[i];
-                d.mode = reqs[i].instance == VC_PVC ? kModePVC : kModeMVC;
-                d.k = std::min<uint32_t>(reqs[i].k, d.n);
-                d.init_best = init_best_for(&reqs[i], d.n);
-                d.node_limit = reqs[i].node_limit;
-                d.m2 = a->row_ptr[a->row_off[i] + d.n];
+                d = desc_of(i);
             }
             d.key = (uint32_t)j;
             tl = std::max(tl, reqs[i].time_limit_s);
         }
         cj.time_limit_s = tl;
         vc_status s = run_job(*c, cj, stream);
-        if (s == VC_OK && check == 2)
-            for (const InstState &st : cj.st)
-                if (st.flags & kBadGraph) return fail(VC_ERR_INVALID);
+        if (s == VC_ERR_INVALID) return fail(s);
         if (s != VC_OK) {
             for (uint32_t i = 0; i < count; ++i) out[i].status = s;
             return s;

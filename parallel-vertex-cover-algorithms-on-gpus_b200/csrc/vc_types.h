@@ -38,6 +38,7 @@ enum : uint32_t {
 enum : unsigned long long {
     kStopTime = 1,  // its time limit
     kStopRing = 2,  // a wait on the ring ran out: a fault of the search, not the caller's limit
+    kStopInput = 3, // a graph of a host-resident call fails its checks: the call is refused
 };
 
 enum : uint32_t { kModeMVC = 0, kModePVC = 1 };
