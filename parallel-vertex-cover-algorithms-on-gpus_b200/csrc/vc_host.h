@@ -223,7 +223,8 @@ Ctx *get_ctx(int dev, vc_status *err);
 cudaError_t make_plan(Ctx &c, uint32_t np, uint32_t nmax, Plan &pl, const PlanOpts &o = PlanOpts());
 void cap_plan(const Ctx &c, Plan &pl, uint32_t per_sm);
 cudaError_t launch_reduce(const ReduceArgs &r, uint32_t ctas, cudaStream_t stream);
-cudaError_t launch_reduce_many(const ReduceArgs *list, uint32_t count, uint32_t ctas, cudaStream_t stream);
+cudaError_t launch_reduce_many(const ReduceArgs *list, uint32_t count, cudaStream_t stream);
+cudaError_t launch_reduce_each(const ReduceArgs *list, uint32_t count, uint32_t nmax, cudaStream_t stream);
 uint32_t reduce_ctas(const Ctx &c);
 vc_status run_job(Ctx &c, Job &job, cudaStream_t stream);
 vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_t n, vc_result *out);

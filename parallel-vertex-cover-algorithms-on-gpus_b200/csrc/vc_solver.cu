@@ -755,39 +755,45 @@ vc_status fill_result(const Job &job, uint32_t i, const vc_request *req, uint32_
 }
 
 // ---------------------------------------------------------------- large graphs
-// How large graphs (largest first) are reduced.  Power-law graphs, measured one at a
-// time (kernel, us; a pass takes the same share of each):
-//   vertices            10,000   30,000   100,000
-//   whole chip             147      178       220
-//   cluster of 8 CTAs      250      503      1330
-//   cluster of 4           340      770      2310
-//   cluster of 2           550     1400      4510
-//   one CTA                955     2570      8520
-// that is 110 us and 46 more for every 512 vertices per CTA; but 37 clusters of 8 (or
-// 296 single CTAs) run side by side, and launches that take the chip one after another.
-// The first `chip` graphs get the chip and the others a cluster each, in the way that
-// these figures make cheapest.  1000 graphs of 1100 to 4000 vertices on the device,
-// planted and power-law: 1.4 and 1.9 ms a call, each with the chip in turn 69 and 125,
-// reduced by the search's own units 2.4 and 2.4; one of 100,000 beside 256 of them
-// 0.65, 17 and 12.
+// How large graphs (largest first) are reduced: the first `chip` by the whole chip, one
+// after another, those up to `near` by a cluster of CTAs each in one launch, the others
+// by one CTA each in another.  Kernel times of one power-law graph, its check included
+// (us; a pass takes the same share of each):
+//   vertices            1,500  3,000  6,000  12,000  24,000  100,000
+//   whole chip            125    116    136     154     167      220
+//   a cluster of 8                              270     380     1330
+//   one CTA                78     82    126     228     416
+// A pass of the chip is two grid barriers and four dependent reads from L2 whatever the
+// size; one CTA's are barriers of its own and shared memory, but it walks all vertices;
+// and 148 CTAs, or 37 clusters, run side by side.  The line between the chip and one
+// CTA for a graph by itself is at 7,400 vertices.  The chip alone (and launches one after
+// another in a batch) had made cascades and batches slower than the search's own units
+// are at a root: a path of 1500 vertices 0.87 -> 2.3 ms, now 0.60; 1000 graphs of 1100
+// to 4000 vertices on the device, planted and power-law, 2.4 -> 69 and 125 ms, now 0.86
+// and 1.3; one of 100,000 vertices beside 256 of them 12 -> 17, now 0.48.
+constexpr uint32_t kNearMax = 24576;  // vertices that one CTA's shared memory holds
 struct ReduceSplit {
-    uint32_t chip, ctas;  // graphs that get the whole chip; CTAs per cluster for the others
+    uint32_t chip, near;
 };
-static ReduceSplit split_reductions(const std::vector<Reduce> &reds, uint32_t resident)
+static ReduceSplit split_reductions(const std::vector<Reduce> &reds, uint32_t sms)
 {
     const uint32_t count = (uint32_t)reds.size();
-    ReduceSplit best{count, 8};
-    if (count == 1) return best;
-    const double chip = 160.0;
-    double sum[4] = {0, 0, 0, 0}, least = chip * count;
-    for (uint32_t k = count; k-- > 0;)  // the first k get the chip
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t ctas = 1u << j;
-            const double one = 110.0 + 46.0 * reds[k].n / (512.0 * ctas);
-            sum[j] += one;
-            const double t = chip * k + std::max(one, sum[j] * ctas / resident);
-            if (t < least) { least = t; best = {k, ctas}; }
-        }
+    uint32_t near = 0;
+    while (near < count && reds[near].n > kNearMax) ++near;
+    ReduceSplit best{count, count};
+    auto on_chip = [](uint32_t n) { return 150.0 + 0.0007 * n; };
+    double chip = 0;
+    for (const Reduce &r : reds) chip += on_chip(r.n);
+    double most[2] = {0, 0}, sum[2] = {0, 0}, least = chip;
+    for (uint32_t k = count; k-- > 0;) {  // the first k get the chip
+        const bool one = k >= near;
+        const double t = one ? 30.0 + 0.0162 * reds[k].n : 110.0 + 0.0112 * reds[k].n;
+        most[one] = std::max(most[one], t);
+        sum[one] += t / (one ? sms : sms / 4);
+        chip -= on_chip(reds[k].n);
+        const double all = chip + std::max(most[0], sum[0]) + std::max(most[1], sum[1]);
+        if (all < least) { least = all; best = {k, std::max(k, near)}; }
+    }
     return best;
 }
 
@@ -799,7 +805,7 @@ static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, co
                                 const std::vector<InstDesc> &others, cudaStream_t stream, float *ms)
 {
     const uint32_t count = (uint32_t)reds.size(), ctas = reduce_ctas(c);
-    const ReduceSplit split = split_reductions(reds, ctas);
+    const ReduceSplit split = split_reductions(reds, (uint32_t)c.sms);
     size_t words = 0;
     auto take = [&](size_t n) {  // 16-byte pieces
         const size_t at = words;
@@ -856,21 +862,29 @@ static vc_status run_reductions(Ctx &c, std::vector<Reduce> &reds, int check, co
     bool ok = cudaMemsetAsync(d_head, 0, count * sizeof(ReduceHead), stream) == cudaSuccess &&
               cudaMemcpyAsync(base, h, 4 * in_words, cudaMemcpyHostToDevice, stream) == cudaSuccess;
     cudaEventRecord(c.ev0, stream);
-    auto check_from = [&](uint32_t i, uint32_t k, uint32_t nmax) {  // graphs i .. i + k - 1 of the list
+    auto check_from = [&](uint32_t i, uint32_t end, uint32_t nmax) {  // graphs i .. end - 1 of the list
+        const uint32_t k = end - i;
         if (!check || k == 0) return;
         ok = ok && launch_check(check == 2, rp, cl, (const InstDesc *)(base + descs) + i, &d_head[check == 2 ? 0 : i].bad,
                                 check == 2 ? 0u : sizeof(ReduceHead) / 4, 1u, k, nmax, stream) == cudaSuccess;
         g_launches += 1;
     };
-    for (uint32_t i = 0; i < split.chip; ++i) check_from(i, 1, reds[i].n);  // a launch's blocks are as many for each of its graphs
-    if (split.chip < count) check_from(split.chip, count - split.chip, reds[split.chip].n);
-    check_from(count, checked - count, others_n);
+    // (a launch's blocks are as many for each of its graphs)
+    for (uint32_t i = 0; i < split.chip; ++i) check_from(i, i + 1, reds[i].n);
+    if (split.chip < split.near) check_from(split.chip, split.near, reds[split.chip].n);
+    if (split.near < count) check_from(split.near, count, reds[split.near].n);
+    check_from(count, checked, others_n);
     for (uint32_t i = 0; ok && i < split.chip; ++i) {
         ok = launch_reduce(reds[i], ctas, stream) == cudaSuccess;
         g_launches += 1;
     }
-    if (split.chip < count) {
-        ok = ok && launch_reduce_many((const ReduceArgs *)(base + list) + split.chip, count - split.chip, split.ctas, stream) == cudaSuccess;
+    const ReduceArgs *d_list = (const ReduceArgs *)(base + list);
+    if (split.chip < split.near) {
+        ok = ok && launch_reduce_many(d_list + split.chip, split.near - split.chip, stream) == cudaSuccess;
+        g_launches += 1;
+    }
+    if (split.near < count) {
+        ok = ok && launch_reduce_each(d_list + split.near, count - split.near, reds[split.near].n, stream) == cudaSuccess;
         g_launches += 1;
     }
     cudaEventRecord(c.ev1, stream);
