@@ -202,6 +202,24 @@ inline bool wide_ok(uint32_t n, const uint32_t *row_ptr)
     return true;
 }
 
+// From how many roots the dense kernels search a graph that has a launch to itself: all
+// n, or one (0), by its size and density (m2 / n^2).
+// At two fifths and above, from 64 vertices, MVC and both PVC answers gain (plain
+// kernel: 200 vertices of 0.5 0.94 -> 0.62 ms, 300 of 0.75 1.65 -> 0.41, 256 of 0.9
+// 0.98 -> 0.09, 1000 of 0.8 6.6 -> 4.1).  Down to 0.15 they do for 16 to 192 vertices:
+// the trees are a few hundred nodes, most of them the spine, and with the packing bound
+// at its nodes they had become slower than without (allocation-free calls, without the
+// bound, with it, and from n roots: 64 vertices of 0.3 0.27, 0.35 and 0.14 ms; of 0.7
+// 0.20, 0.31 and 0.07; 180 vertices, bipartite, PVC no 0.33, 0.38 and 0.16).  Above that
+// size the spine is a small part of the tree at 0.3 (200 vertices 6.2 -> 5.8) and a PVC
+// "yes", which the first descent often finds, comes later (0.8 -> 1.6).
+inline uint32_t split_roots(uint32_t n, uint32_t m2)
+{
+    const uint64_t n2 = (uint64_t)n * n;
+    if (m2 == vcg::kNone) return 0u;
+    return (n >= 64 && 5ull * m2 >= 2 * n2) || (n >= 16 && n <= 192 && 20ull * m2 >= 3 * n2) ? n : 0u;
+}
+
 struct PlanOpts {
     uint32_t smem_budget = 0;  // bytes per CTA for CSR workspaces, 0 = the device limit
     uint32_t warp_max_np = 0;  // largest capacity given warp units, 0 = kWarpMaxNP

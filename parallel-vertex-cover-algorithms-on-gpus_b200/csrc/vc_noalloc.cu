@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dense_noalloc(Params P)
 }
 
 // Clears the shared array for a new call and writes the graph's descriptor.
-__global__ void k_noalloc_reset(Scratch *s, InstDesc d)
+__global__ void k_noalloc_reset(Scratch *s, InstDesc d, uint32_t roots)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kRingSlots) s->seq[i] = i;
@@ -87,7 +87,7 @@ __global__ void k_noalloc_reset(Scratch *s, InstDesc d)
         s->desc = d;
         InstState st;
         st.best = d.init_best;
-        st.act = 1;
+        st.act = roots;
         st.flags = 0;
         st.lock = 0;
         st.cover_size = kNone;
@@ -237,8 +237,10 @@ extern "C" vc_status vc_solve_noalloc(const vc_csr *g, const vc_request *req, ui
     // Launches are checked through their own return codes, so an error the
     // caller's earlier work left pending is neither reported nor cleared here.
     Scratch *s = su->scratch;
+    const uint32_t split = vch::split_roots(n, d.m2);
     {
-        void *a[] = {&s, &d};
+        uint32_t roots = split ? split : 1u;
+        void *a[] = {&s, &d, &roots};
         if (cudaLaunchKernel((const void *)k_noalloc_reset, dim3((kRingSlots + 255) / 256), dim3(256), a, 0, stream) !=
             cudaSuccess)
             return VC_ERR_CUDA;
@@ -251,7 +253,7 @@ extern "C" vc_status vc_solve_noalloc(const vc_csr *g, const vc_request *req, ui
         uint32_t *flags = &s->st.flags;
         uint32_t stride = 1, value = kBadGraph, one = 1, *mate = nullptr;
         void *a[] = {&rp, &cl, &di, &flags, &stride, &value, &one, &mate};
-        if (cudaLaunchKernel((const void *)k_check_csr<false>, dim3(1), dim3(256), a, 0, stream) != cudaSuccess)
+        if (cudaLaunchKernel((const void *)k_check_csr<false>, dim3(1, (n + 7) / 8), dim3(256), a, 0, stream) != cudaSuccess)
             return VC_ERR_CUDA;
     }
 
@@ -276,6 +278,7 @@ extern "C" vc_status vc_solve_noalloc(const vc_csr *g, const vc_request *req, ui
     P.stats = nullptr;
     const double tl = req->time_limit_s > 0 ? req->time_limit_s : 300.0;
     P.time_limit_ns = (unsigned long long)(tl * 1e9);
+    P.split = split;
     void *args[] = {&P};
     const void *fn = idx == 0 ? (const void *)k_dense_noalloc<2, 256>
                               : (idx == 1 ? (const void *)k_dense_noalloc<4, 256> : (const void *)k_dense_noalloc<8, 256>);

@@ -519,18 +519,6 @@ static unsigned long long pack_after(const InstDesc &d)
     return d.n > 128 && d.n <= 255 && d.m2 != kNone && d.m2 >= 2 * 768 ? 25000000ull : 0ull;
 }
 
-// From how many roots a plain solve's dense kernel searches the graph: all n, for
-// graphs of 64 vertices or more whose average degree is at least two fifths of n; else
-// one (0).  Measured at densities 0.5 and up, MVC and both PVC answers gain (kernel:
-// 200 vertices of 0.5 0.94 -> 0.62 ms, 300 of 0.75 1.65 -> 0.41, 256 of 0.9 0.98 ->
-// 0.09, 1000 of 0.8 6.6 -> 4.1); at 0.3 the spine is a small part of the tree (200
-// vertices 6.2 -> 5.8) and a PVC "yes", which the first descent often finds, comes
-// later (0.8 -> 1.6).
-static uint32_t split_roots(const InstDesc &d)
-{
-    return d.n >= 64 && d.m2 != kNone && 5ull * d.m2 >= 2ull * d.n * d.n ? d.n : 0u;
-}
-
 // ---------------------------------------------------------------- one launch
 // Runs every graph of `job` (arena already on the device) to completion and
 // copies back the per-graph state and cover bitmaps.
@@ -616,7 +604,7 @@ vc_status run_job(Ctx &c, Job &job, cudaStream_t stream)
     A.st = (InstState *)(d_out + st_at);
     A.inst = (const InstDesc *)d_in;
     A.count = count;
-    const uint32_t split = count == 1 && nw ? split_roots(job.desc[0]) : 0u;
+    const uint32_t split = count == 1 && nw ? split_roots(job.desc[0].n, job.desc[0].m2) : 0u;
     A.roots = split ? split : 1u;
     A.row_ptr = job.d_rp;
     A.col = job.d_col;
