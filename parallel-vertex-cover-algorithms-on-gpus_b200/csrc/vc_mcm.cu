@@ -59,6 +59,18 @@ struct McmArgs {
 // descent is one unit's (planted matching of 1024 vertices 0.45 -> 0.32 ms).
 constexpr uint32_t kMcmRowBytes = 64u << 10;
 
+// A word of the rows.  Rows left in global memory (Far) have a kernel of their own, which
+// reads them through the read-only path: complete graphs of 200 and 1024 vertices 0.53
+// and 12.6 ms, with one kernel for both 0.58 and 14.6.  The other keeps its generic
+// pointers: with plain shared-memory reads the first descent came out slower (planted
+// matchings of 255 and 1024 vertices 0.17 -> 0.22 and 0.42 -> 0.47 ms).
+template <bool Far>
+__device__ __forceinline__ uint32_t mcm_word(const uint32_t *p)
+{
+    if constexpr (Far) return __ldg(p);
+    else return *p;
+}
+
 // Frame depth of one unit: at most n/2 matched entries, plus one.
 __host__ __device__ inline uint32_t mcm_depth(uint32_t n) { return n / 2 + 1; }
 
@@ -75,6 +87,7 @@ __device__ __forceinline__ uint32_t mcm_next_row(uint32_t av, uint32_t r, uint32
 
 // The first entry at or after (cr, ce) whose row and column vertices are both
 // available (findNextEdgeByWarp's choice); false if none is left.
+template <bool Far>
 __device__ __forceinline__ bool mcm_next_entry(const uint32_t *rp, const uint32_t *cl, uint32_t n, uint32_t av,
                                                uint32_t lane, uint32_t cr, uint32_t ce, uint32_t &er, uint32_t &ee)
 {
@@ -82,11 +95,11 @@ __device__ __forceinline__ bool mcm_next_entry(const uint32_t *rp, const uint32_
     for (;;) {
         const uint32_t nr = mcm_next_row(av, r, lane);
         if (nr == kNone || nr >= n) return false;
-        const uint32_t e0 = nr == cr ? max(ce, rp[nr]) : rp[nr];
-        const uint32_t e1 = rp[nr + 1];
+        const uint32_t e0 = nr == cr ? max(ce, mcm_word<Far>(&rp[nr])) : mcm_word<Far>(&rp[nr]);
+        const uint32_t e1 = mcm_word<Far>(&rp[nr + 1]);
         for (uint32_t eb = e0; eb < e1; eb += 32) {
             const uint32_t ei = eb + lane;
-            const uint32_t u = ei < e1 ? cl[ei] : 0u;
+            const uint32_t u = ei < e1 ? mcm_word<Far>(&cl[ei]) : 0u;
             const uint32_t word = __shfl_sync(0xffffffffu, av, u >> 5);
             const uint32_t b = __ballot_sync(0xffffffffu, ei < e1 && ((word >> (u & 31u)) & 1u));
             if (b) {
@@ -190,7 +203,7 @@ __global__ void k_mcm_init_ring(unsigned long long *seq, uint32_t q)
     if (i < q) seq[i] = i;
 }
 
-template <unsigned NT>
+template <unsigned NT, bool Far>
 __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
 {
     extern __shared__ __align__(16) uint32_t msm[];
@@ -200,7 +213,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
     uint32_t *fp = fe + depth;                       // its row | column << 16
     InstState &st = P.st[0];
     const uint32_t *rp = P.row_ptr, *cl = P.col;
-    if (A.rows_in) {
+    if (!Far && A.rows_in) {
         uint32_t *rows = msm + (size_t)(NT / 32) * 2u * depth;
         for (uint32_t i = threadIdx.x; i <= A.n; i += NT) rows[i] = __ldg(&rp[i]);
         for (uint32_t i = threadIdx.x; i < A.m2; i += NT) rows[A.n + 1 + i] = __ldg(&cl[i]);
@@ -217,7 +230,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
     if (su == 0) {  // the root: every vertex with a neighbour, cursor at entry 0
         for (uint32_t b = 0; b < 32; ++b) {
             const uint32_t v = 32u * lane + b;
-            if (v < A.n && rp[v + 1] > rp[v]) av |= 1u << b;
+            if (v < A.n && mcm_word<Far>(&rp[v + 1]) > mcm_word<Far>(&rp[v])) av |= 1u << b;
         }
         have = true;
     }
@@ -265,7 +278,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
         uint32_t er = 0, ee = 0;
         bool descend = false;
         if (cnt < A.n && c_best < A.n && cnt + (avc & ~1u) > c_best)
-            descend = mcm_next_entry(rp, cl, A.n, av, lane, cr, ce, er, ee);
+            descend = mcm_next_entry<Far>(rp, cl, A.n, av, lane, cr, ce, er, ee);
         if (!descend && cnt > c_best) {
             // a leaf (every vertex unavailable, or no eligible entry left; a cut subtree
             // cannot count more than the maximum): raise the maximum
@@ -285,7 +298,7 @@ __global__ void __launch_bounds__(NT) k_mcm(Params P, McmArgs A)
                 bot += 1;
                 c_state += 1ull << 32;
             }
-            const uint32_t u = cl[ee];
+            const uint32_t u = mcm_word<Far>(&cl[ee]);
             if (lane == 0) {
                 fe[level] = ee;
                 fp[level] = er | (u << 16);
@@ -357,7 +370,7 @@ extern "C" vc_status vc_mcm(const vc_csr *g, const vc_request *req, vc_result *o
     const uint64_t row_bytes = 4ull * (n + 1 + (uint64_t)m2);
     const bool rows_in = row_bytes <= kMcmRowBytes;
     const uint32_t smem = (kMcmThreads / 32) * 2u * mcm_depth(n) * 4u + (rows_in ? (uint32_t)row_bytes : 0u);
-    auto fn = k_mcm<kMcmThreads>;
+    auto fn = rows_in ? k_mcm<kMcmThreads, false> : k_mcm<kMcmThreads, true>;
     int per_sm = 0;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)kMcmThreads, smem) != cudaSuccess ||

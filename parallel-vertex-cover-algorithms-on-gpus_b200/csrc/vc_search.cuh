@@ -696,10 +696,13 @@ __device__ __forceinline__ bool ring_wait(const Params &P, unsigned long long po
 {
     for (int it = 0; it < kRingSpins; ++it) {
         if (ld_acquire_u64(&P.pool_seq[pos & P.q_mask]) == seq) return true;
-        if ((it & 255) == 255 && ld_relaxed_u64(&P.ctl[kAbort])) return false;
         __nanosleep(32);
+        if ((it & 255) == 255 && ld_relaxed_u64(&P.ctl[kAbort])) break;
     }
-    stop_launch(P, kStopRing);
+    // a launch that something else has stopped keeps its reason.  (One way out of the loop
+    // that fails: with two the compiler made the wait a call and gave k_mcm 32 registers
+    // instead of 40.)
+    atomicCAS(&P.ctl[kAbort], 0ull, (unsigned long long)kStopRing);
     return false;
 }
 
