@@ -27,7 +27,7 @@
 //    failed test succeed; so a test that failed can only succeed once i is dirty or
 //    its second neighbour's row has moved.  The first firing vertex in index order
 //    is the one the reference's restart-from-zero sweep would reach first.
-//  * the largest degree (RemoveMax): an upper bound per 1024 vertices, made exact
+//  * the largest degree (RemoveMax): an upper bound per block of vertices, made exact
 //    only where it is the largest of all -- degrees only fall.
 // The reference's binary search (auxFunctions.cpp:25-42) steps an unsigned
 // index below zero (and reads out of bounds) in one corner case; there this
@@ -85,7 +85,7 @@ struct UbParams {
     uint32_t r;        // RemoveEdge: the value of rand() the reference's draws used
 };
 
-constexpr uint32_t kMaxBlock = 1024;  // vertices per cached maximum
+constexpr int kShortRow = 8;          // entries of a moved row that one thread looks through
 constexpr int kWarpDelete = 96;       // neighbours up to which one warp deletes a leaf's neighbour
 
 // deg1, two, dirty, moved and deg1's summary, in words; then the cached maxima (two
@@ -95,7 +95,21 @@ __host__ __device__ inline uint64_t ub_bitmap_words(uint32_t n)
     const uint64_t nw = (n + 31) / 32;
     return (4 * nw + (nw + 31) / 32 + 1) / 2 * 2;
 }
-__host__ __device__ inline uint64_t ub_set_words(uint32_t n) { return ub_bitmap_words(n) + 2ull * ((n + kMaxBlock - 1) / kMaxBlock); }
+// A cached maximum is of 2^shift vertices.  Graphs of up to 8192 vertices have as many
+// blocks as the CTA has warps, at most, and each warp makes its block's maximum anew;
+// above, about as many blocks as vertices in one, which one warp looks through.  (1024
+// each: RemoveMax on 3-regular graphs of 1000 and 16,000 vertices 1.90 and 40.1 ms; with
+// this and the moved rows' vertices marked 1.35 and 28.6.)
+__host__ __device__ inline uint32_t ub_max_shift(uint32_t n)
+{
+    uint32_t s = 7;
+    while (s < 9 && ((uint64_t)kUbWarps << s) < n) ++s;
+    if (((uint64_t)kUbWarps << s) >= n) return s;
+    for (s = 7; s < 16 && (1ull << (2 * s)) < n;) ++s;
+    return s;
+}
+__host__ __device__ inline uint32_t ub_max_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n + (1u << ub_max_shift(n)) - 1) >> ub_max_shift(n)); }
+__host__ __device__ inline uint64_t ub_set_words(uint32_t n) { return ub_bitmap_words(n) + 2ull * ub_max_blocks(n); }
 __host__ __device__ inline uint64_t ub_all_words(uint32_t n) { return ub_set_words(n) + 4ull * n + 1; }
 
 struct UbShared {
@@ -114,8 +128,8 @@ struct Ub {
     uint2 *gone;
     int32_t *deg;
     uint32_t *d1, *s1, *d2, *dt, *mv;  // deg1, its summary, two, dirty, moved
-    unsigned long long *bmax;          // per kMaxBlock vertices: at least the largest key
-    uint32_t n, nw;
+    unsigned long long *bmax;          // per 2^shift vertices: at least the largest key
+    uint32_t n, nw, shift;
 };
 
 __device__ __forceinline__ unsigned lane_of() { return threadIdx.x & 31u; }
@@ -236,7 +250,7 @@ __device__ uint32_t ub_next_leaf(const Ub &g, uint32_t p)
 __device__ unsigned long long ub_block_max(const Ub &g, uint32_t i)
 {
     unsigned long long best = 0;
-    const uint32_t lo = i * kMaxBlock, hi = min(g.n, lo + kMaxBlock);
+    const uint32_t lo = i << g.shift, hi = min(g.n, lo + (1u << g.shift));
     for (uint32_t v = lo + lane_of(); v < hi; v += 32) {
         const int d = g.deg[v];
         const unsigned long long key = d > 0 ? ((unsigned long long)(uint32_t)d << 32) | (uint32_t)(~v) : 0ull;
@@ -296,6 +310,7 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
     Ub g;
     g.n = n;
     g.nw = (n + 31) / 32;
+    g.shift = ub_max_shift(n);
     g.dst = P.dst + col_off;
     g.mate = P.mate + col_off;
     g.gone = P.gone + row_off;
@@ -325,15 +340,22 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
     if (all_in)
         for (uint32_t v = threadIdx.x; v <= n; v += kUbThreads) rp_in[v] = rp0[v];
     __syncthreads();
+    // With no row of more than kShortRow entries the triangle rule marks the degree-2
+    // vertices of the rows that have moved; else every degree-2 vertex looks at its second
+    // neighbour, as deletions beside long rows move too many of them (G(2000, 0.5) 12.5
+    // ms, marked 17.3; but on a 3-regular graph of 4000 vertices RemoveMax and RemoveEdge
+    // took 6.2 and 5.1, marked 5.2 and 4.5).
+    bool is_long = false;
     for (uint32_t v = threadIdx.x; v < n; v += kUbThreads) {
         const int d = (int)(g.rp[v + 1] - g.rp[v]);
+        is_long = is_long || d > kShortRow;
         g.deg[v] = d;
         g.gone[v] = make_uint2(0u, 0u);
         if (d == 1) ub_set1(g, sh, v);
         if (d == 2) ub_put(g.d2, v);
     }
-    __syncthreads();
-    const uint32_t blocks = (n + kMaxBlock - 1) / kMaxBlock;
+    const bool all_short = !__syncthreads_or(is_long);
+    const uint32_t blocks = ub_max_blocks(n);
     if (P.mode == 0)
         for (uint32_t i = warp_of(); i < blocks; i += kUbWarps) {
             const unsigned long long k = ub_block_max(g, i);
@@ -394,6 +416,24 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
         for (;;) {
             __syncthreads();
             if (!sh.any) break;
+            if (all_short) {  // the degree-2 vertices of moved rows are due, and no others
+                for (uint32_t wi = threadIdx.x; wi < g.nw; wi += kUbThreads) {
+                    uint32_t m = g.mv[wi];
+                    if (m) g.mv[wi] = 0;
+                    while (m) {
+                        const uint32_t v = 32u * wi + (uint32_t)(__ffs(m) - 1);
+                        m &= m - 1;
+                        const int d = g.deg[v];
+                        uint32_t y[kShortRow];
+#pragma unroll
+                        for (int k = 0; k < kShortRow; ++k) y[k] = k < d ? g.dst[g.rp[v] + k] : v;
+#pragma unroll
+                        for (int k = 0; k < kShortRow; ++k)
+                            if (k < d && ub_has(g.d2, y[k])) ub_put(g.dt, y[k]);
+                    }
+                }
+                __syncthreads();
+            }
             uint32_t fire = kInf;
             for (uint32_t base = 0; base < g.nw && fire == kInf; base += kUbThreads) {
                 __syncthreads();
@@ -403,6 +443,7 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
                 if (wi < g.nw) {
                     uint32_t x = g.d2[wi];
                     const uint32_t fresh = g.dt[wi];
+                    if (all_short) x &= fresh;
                     while (x) {
                         const uint32_t i = 32u * wi + (uint32_t)(__ffs(x) - 1);
                         x &= x - 1;
@@ -436,9 +477,24 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
             minimum += 2;
         }
         if (P.mode == 0) {
-            // the lowest-index vertex of maximum degree: the largest cached maximum
-            // that is still exact
-            for (;;) {
+            // the lowest-index vertex of maximum degree
+            unsigned long long k = 0;
+            if (blocks <= kUbWarps) {
+                __syncthreads();
+                if (warp_of() < blocks) {
+                    const unsigned long long now = ub_block_max(g, warp_of());
+                    if (lane_of() == 0) g.bmax[warp_of()] = now;
+                }
+                __syncthreads();
+                k = lane_of() < blocks ? g.bmax[lane_of()] : 0ull;
+#pragma unroll
+                for (int j = 16; j; j >>= 1) {
+                    const unsigned long long o = __shfl_xor_sync(0xffffffffu, k, j);
+                    k = o > k ? o : k;
+                }
+            }
+            // the largest cached maximum that is still exact
+            else for (;;) {
                 __syncthreads();
                 if (warp_of() == 0) {
                     unsigned long long best = 0;
@@ -461,9 +517,9 @@ __global__ void __launch_bounds__(kUbThreads) k_ub(UbParams P)
                     }
                 }
                 __syncthreads();
+                k = sh.amax;
                 if (sh.found) break;
             }
-            const unsigned long long k = sh.amax;
             if (k == 0) break;
             ub_delete<false>(g, sh, ~(uint32_t)k, stamp);
             minimum += 1;
@@ -594,7 +650,7 @@ vc_status ub_run(const vc_csr_arena *a, uint32_t mode, uint32_t r, int32_t devic
     P.mode = mode;
     P.r = r;
     // shared memory for the largest graph that fits whole; graphs above keep what fits of theirs
-    const uint64_t room = (uint64_t)c->smem_optin - sizeof(UbShared) - 1024;
+    const uint64_t room = (uint64_t)c->smem_optin - sizeof(UbShared) - 256;
     uint64_t need = 0;
     for (uint32_t i = 0; i < count; ++i)
         for (const uint64_t w : {ub_set_words(a->n[i]), ub_all_words(a->n[i])})
