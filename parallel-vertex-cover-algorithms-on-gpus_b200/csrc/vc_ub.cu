@@ -565,13 +565,6 @@ vc_status ub_run(const vc_csr_arena *a, uint32_t mode, uint32_t r, int32_t devic
     uint32_t nmax = 0;
     std::vector<uint64_t> boff(count);
     std::vector<InstDesc> desc(count);
-    for (uint32_t i = 0; i < count; ++i) {
-        if (a->n[i] > kMaxVertices) return VC_ERR_TOO_LARGE;
-        nmax = std::max(nmax, a->n[i]);
-        rows = std::max<uint64_t>(rows, a->row_off[i] + a->n[i] + 1);
-        boff[i] = bits;
-        bits += ub_set_words(a->n[i]);
-    }
     auto graph = [&](uint32_t i) {
         const uint32_t *rp = a->row_ptr + a->row_off[i];
         vc_csr g;
@@ -582,6 +575,19 @@ vc_status ub_run(const vc_csr_arena *a, uint32_t mode, uint32_t r, int32_t devic
         g.degree = nullptr;
         return g;
     };
+    for (uint32_t i = 0; i < count; ++i) {
+        if (a->n[i] > kMaxVertices) {  // unless a graph before it is invalid
+            for (uint32_t j = 0; j < i; ++j) {
+                const vc_csr g = graph(j);
+                if (validate_csr(&g) != VC_OK) return VC_ERR_INVALID;
+            }
+            return VC_ERR_TOO_LARGE;
+        }
+        nmax = std::max(nmax, a->n[i]);
+        rows = std::max<uint64_t>(rows, a->row_off[i] + a->n[i] + 1);
+        boff[i] = bits;
+        bits += ub_set_words(a->n[i]);
+    }
     for (uint32_t i = 0; i < count; ++i) {
         const vc_csr g = graph(i);
         const vc_status v = check_head(&g);
